@@ -327,35 +327,37 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
             __syncwarp();
             bool emit_node = false, emit_range = false, push = false;
             uint32_t r0 = 0, r1 = 0;
-            float4 mom = make_float4(0.f, 0.f, 0.f, 0.f), sq = mom;
             if (has) {
                 if (v >= nm1) {
                     emit_range = true;
                     r0 = v - nm1;
                     r1 = 1;
                 } else {
-                    const float4 box = __ldg(&gnode[v].box);
-                    const uint4 lk = __ldg(&gnode[v].link);
-                    mom = __ldg(&gnode[v].mom);
-                    if (MP >= 2) sq = __ldg(&gnode[v].quad);
-                    if (group_accepts(box, mom.x, mom.y, glox, gloy, ghix, ghiy, th2)) {
+                    float4 box, tr;
+                    ldg_half(&gnode[v].box, box, tr);
+                    const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
+                    if (group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2)) {
                         emit_node = true;
-                    } else if (lk.w <= (uint32_t)P.leaf_size) {
+                    } else if ((small & 255u) <= (uint32_t)P.leaf_size) {
                         emit_range = true;
-                        r0 = lk.z;
-                        r1 = lk.w;
+                        r0 = link_gamma(link) + 1u - (small >> 8);
+                        r1 = small & 255u;
                     } else {
                         push = true;
-                        r0 = lk.x;
-                        r1 = lk.y;
+                        r0 = link_left(link, nm1);
+                        r1 = link_right(link, nm1);
                     }
                 }
             }
             const unsigned mn = __ballot_sync(FULL, emit_node);
             if (emit_node) {
                 const int p = nn + __popc(mn & lt);
-                const float tr = sq.x + sq.z;  // Q' = 3S - tr(S) I
-                const float qxx = 3.0f * sq.x - tr, qxy = 3.0f * sq.y, qyy = 3.0f * sq.z - tr;
+                float4 mom, tail;  // {com, mass, Sxx}, {Sxy, Syy}
+                ldg_half(&gnode[v].mom, mom, tail);
+                const float sxx = MP >= 2 ? mom.w : 0.f, sxy = MP >= 2 ? tail.x : 0.f;
+                const float syy = MP >= 2 ? tail.y : 0.f;
+                const float tr = sxx + syy;  // Q' = 3S - tr(S) I
+                const float qxx = 3.0f * sxx - tr, qxy = 3.0f * sxy, qyy = 3.0f * syy - tr;
                 S.nd[p][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
                 S.nd[p][1] = make_float4(mom.z, mom.z, qxx, qxx);
                 S.nd[p][2] = make_float4(qxy, qxy, qyy, qyy);

@@ -48,15 +48,44 @@ constexpr uint32_t kDebugLookbackUnpublished = 1u << 0;
 // the split hierarchy build (local phase + frontier climb) at every body count from 2
 constexpr uint32_t kDebugSplitBuild = 1u << 1;
 
-// Packed internal-node record of the group walk (64 B, one per internal node):
-// the criterion reads `box`, an accepted node contributes `mom` + `quad`, an
-// opened node continues through `link`.
-struct __align__(16) GNode {
-    float4 box;   // {min.x, min.y, max.x, max.y}
-    float4 mom;   // {com.x, com.y, mass, length}
-    float4 quad;  // raw second moments about the COM {Sxx, Sxy, Syy, 0}
-    uint4 link;   // {left, right, first slot, body count}
+// Packed internal-node record of the group walk (64 B, one per internal node),
+// in two 32-B halves (a sector each, one 256-bit load): what an accepted node
+// contributes, and what the traversal reads to accept or open it.
+struct __align__(32) GNode {
+    float4 mom;  // {com.x, com.y, mass, Sxx}: S = raw second moments about the COM
+    float4 tail; // {Sxy, Syy, first slot (bits), body count (bits)}
+    float4 box;  // {min.x, min.y, max.x, max.y}
+    float4 trav; // {com.x, com.y, link (bits), small (bits)}
 };
+// trav.z: the split gamma (30 bits) and which children are leaves; in the
+// Karras numbering the children are gamma / gamma + 1 or the leaves
+// n-1+gamma / n+gamma.  trav.w: body count and left child's body count, 255
+// for more (the traversal compares counts with a leaf size of at most 8).
+constexpr uint32_t kLinkLeftLeaf = 1u << 30, kLinkRightLeaf = 1u << 31;
+__host__ __device__ __forceinline__ uint32_t link_gamma(uint32_t link) { return link & 0x3FFFFFFFu; }
+__host__ __device__ __forceinline__ uint32_t link_left(uint32_t link, uint32_t nm1) {
+    return link_gamma(link) + (link & kLinkLeftLeaf ? nm1 : 0u);
+}
+__host__ __device__ __forceinline__ uint32_t link_right(uint32_t link, uint32_t nm1) {
+    return link_gamma(link) + 1u + (link & kLinkRightLeaf ? nm1 : 0u);
+}
+__host__ __device__ __forceinline__ uint32_t pack_small(uint32_t count, uint32_t lcount) {
+    return (count < 255u ? count : 255u) | ((lcount < 255u ? lcount : 255u) << 8);
+}
+
+// 256-bit accesses to one 32-B half (32-B aligned).  A gathered load of a whole
+// half costs the L1 one pass over the warp's 32 lines where two 128-bit loads
+// cost two.
+__device__ __forceinline__ void ldg_half(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+__device__ __forceinline__ void st_half(float4* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x),
+                 "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 
 // Group acceptance test.  A node stands in for its bodies, as one multipole,
 // for a whole group when its size L and the distance d from the group's box
@@ -90,10 +119,7 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// Group-walk stack and list capacities (per warp).
-constexpr int kGroupStack = 1024;
-constexpr int kGroupDfsAt = kGroupStack - 128;  // switch to one node per step above this depth
-constexpr int kGroupList = 64;
+constexpr int kGroupList = 64;  // node list of the group walk and its VJP (per warp)
 constexpr int kGroupMaxLeaf = 8;                // leaf_size cap of the group walk
 constexpr uint32_t kErrGroupStack = 1u << 3;    // group-walk stack overflow (never expected)
 constexpr uint32_t kErrShardCapacity = 1u << 4; // a shard's updated range exceeded its chunk

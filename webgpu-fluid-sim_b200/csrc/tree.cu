@@ -88,11 +88,15 @@ ref_layout_kernel(const GNode* __restrict__ gnode, uint32_t ni, float4* __restri
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < ni; v += gridDim.x * blockDim.x) {
         const float4 box = __ldg(&gnode[v].box);
         const float4 mom = __ldg(&gnode[v].mom);
-        const uint4 lk = __ldg(&gnode[v].link);
-        node4[v] = mom;
+        const float4 tail = __ldg(&gnode[v].tail);
+        const uint32_t link = __float_as_uint(__ldg(&gnode[v].trav.z));
+        const uint32_t first = __float_as_uint(tail.z), count = __float_as_uint(tail.w);
+        // length = longest side, as the build computed it for the reference layout
+        node4[v] = make_float4(mom.x, mom.y, mom.z,
+                               fmaxf(__fsub_rn(box.z, box.x), __fsub_rn(box.w, box.y)));
         aabb[v] = box;
-        children[v] = make_uint2(lk.x, lk.y);
-        range[v] = make_uint2(lk.z, lk.z + lk.w - 1u);
+        children[v] = make_uint2(link_left(link, ni), link_right(link, ni));
+        range[v] = make_uint2(first, first + count - 1u);
     }
 }
 

@@ -309,7 +309,8 @@ __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c, Buil
         } else if (A.gnode) {
             sb = __ldcg(&A.gnode[sib].box);
             s4 = __ldcg(&A.gnode[sib].mom);
-            sq = __ldcg(&A.gnode[sib].quad);
+            const float4 st = __ldcg(&A.gnode[sib].tail);
+            sq = make_float4(s4.w, st.x, st.y, 0.f);
         } else {
             s4 = __ldcg(&A.node4[sib]);
             sb = __ldcg(&A.aabb[sib]);
@@ -394,12 +395,13 @@ __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c, Buil
             c.sxx = __fadd_rn(__fmaf_rn(madx, dax, sax), __fmaf_rn(mbdx, dbx, sbx));
             c.sxy = __fadd_rn(__fmaf_rn(madx, day, say), __fmaf_rn(mbdx, dby, sby));
             c.syy = __fadd_rn(__fmaf_rn(mady, day, saz), __fmaf_rn(mbdy, dby, sbz));
-            GNode g;
-            g.box = make_float4(c.lox, c.loy, c.hix, c.hiy);
-            g.mom = make_float4(ncx, ncy, tm, len);
-            g.quad = make_float4(c.sxx, c.sxy, c.syy, 0.0f);
-            g.link = make_uint4(li, ri, pl, cnt);
-            A.gnode[pidx] = g;
+            GNode* const g = &A.gnode[pidx];
+            const uint32_t link = gamma | (li >= nm1 ? kLinkLeftLeaf : 0u) | (ri >= nm1 ? kLinkRightLeaf : 0u);
+            st_half(&g->mom, make_float4(ncx, ncy, tm, c.sxx),
+                    make_float4(c.sxy, c.syy, __uint_as_float(pl), __uint_as_float(cnt)));
+            st_half(&g->box, make_float4(c.lox, c.loy, c.hix, c.hiy),
+                    make_float4(ncx, ncy, __uint_as_float(link),
+                                __uint_as_float(pack_small(cnt, gamma - pl + 1u))));
         }
         if (A.groups) {
             // Walk groups: maximal subtrees of <= gmax bodies.  A child is one
@@ -600,8 +602,8 @@ build_climb_kernel(const BuildArgs<K> A) {
             if (A.gnode) {
                 box = A.gnode[idx].box;
                 mom = A.gnode[idx].mom;
-                const float4 q = A.gnode[idx].quad;
-                c.sxx = q.x; c.sxy = q.y; c.syy = q.z;
+                const float4 q = A.gnode[idx].tail;
+                c.sxx = mom.w; c.sxy = q.x; c.syy = q.y;
             } else {
                 box = A.aabb[idx];
                 mom = A.node4[idx];

@@ -33,8 +33,8 @@
 // evaluated when they hold >= 32 entries: every lane runs every entry for its
 // BPL bodies (shared-memory broadcasts, no divergence); body records are
 // first loaded 32 at a time by the 32 lanes in parallel.
-// Above kGroupDfsAt entries the warp pops one node per step (plain DFS), which
-// keeps the stack below kGroupStack for any tree of depth <= 96; a push that
+// Above kWalkDfsAt entries the warp pops one node per step (plain DFS), which
+// keeps the stack below kWalkStack for any tree of depth <= 96; a push that
 // would not fit raises kErrGroupStack instead of writing out of bounds.
 // Groups are taken from an atomic counter (the walk is persistent).
 //
@@ -59,47 +59,39 @@
 
 namespace bh {
 
-// Per-warp stack entries.  Shared memory and L1 share each SM's 256 KB, so
-// every byte of stack is L1 the node records lose: 320 entries instead of
-// 384 put 6 far-field blocks per SM in a 196 KB carve-out instead of 228
-// (16.8M bodies: walk 7.67 -> 7.50 ms).  256 entries were slower (0.391 ->
-// 0.407 ms at 800k): more warps reach the one-node-per-step depth guard.
+// Per-warp stack entries.  256 entries were slower (0.391 -> 0.407 ms at 800k):
+// more warps reach the one-node-per-step depth guard.
 constexpr int kWalkStack = 320;
 constexpr int kWalkDfsAt = kWalkStack - 128;  // >= 32 + 96 below the capacity
 
 constexpr int kSlotList = 32 + 32 * kGroupMaxLeaf;  // body slots: < 32 kept + one step's adds
-// Node list entries.  Without the far field the multipole list is flushed
-// at 32 entries, so it holds < 64 after any step.  With it, multipole
-// entries grow from the bottom and far entries from the top; both lists are
-// flushed at 32 entries, so before a step each holds < 32 and one step adds
-// at most 32 in all: < 96 together.
-template <bool FAR>
+// A warp's shared memory.  The lists hold node ids and slots: a step adds at
+// most 32 ids to fewer than 32 kept ones.  Nodes and bodies are staged 32 at a
+// time for their evaluation.
 struct GroupSmem {
-    static constexpr int kListCap = FAR ? 96 : kGroupList;
     uint32_t stack[kWalkStack];
-    // node entry j: ent[j][0] = {cx, cx, cy, cy}, ent[j][1] = {m, m, -Q'xx, -Q'xx},
-    //               ent[j][2] = {-Q'xy, -Q'xy, -Q'yy, -Q'yy}
-    // far entry j (at kListCap - 1 - j): {cx, cy, m, Sxx}, {Sxy, Syy, 0, 0}
-    float4 ent[kListCap][3];
+    // staged node j: ent[j][0] = {cx, cx, cy, cy}, ent[j][1] = {m, m, -Q'xx, -Q'xx},
+    //                ent[j][2] = {-Q'xy, -Q'xy, -Q'yy, -Q'yy}
+    float4 ent[32][3];
+    float4 body[32][2];        // staged leaf records as pairs {x,x,y,y}, {m,m,0,0}
+    uint32_t near[64];         // nodes to evaluate at each body
+    uint32_t far[64];          // nodes for the group's local expansion
     uint32_t slot[kSlotList];  // sorted slots of bodies to sum one by one
-    float4 body[32][2];        // 32 staged leaf records as pairs {x,x,y,y}, {m,m,0,0}
 };
 
-// Far list: the top `cnt` (<= 32) far entries of `nf_total`, one per lane,
-// added to the lane's local-expansion sums.  Not inlined: the coefficient
-// arithmetic is the walk's register peak, and as a call (the caller's live
-// values saved around it, the sums in a 56-B stack frame) the 128-body
-// far-field walk fits 6 blocks per SM in 80 registers instead of 5 in 96.
-// A call costs little once per 32 far nodes (800k bodies: walk 0.399 ->
-// 0.392 ms; 16.8M: 7.87 -> 7.69 ms).
-__device__ __noinline__ void far_batch(GroupSmem<true>& S, float (&cacc)[kFarCoeffs], int lane,
-                                          int nf_total, int cnt, float gcx, float gcy, float lam,
-                                          float eps2) {
-    constexpr int cap = GroupSmem<true>::kListCap;
+// Far list: one node per lane (lane < cnt) added to the lane's local-expansion
+// sums.  Not inlined: the coefficient arithmetic is the walk's register peak,
+// and as a call (the caller's live values saved around it, the sums in a 56-B
+// stack frame) the 128-body far-field walk fits 6 blocks per SM in 80
+// registers instead of 5 in 96.  A call costs little once per 32 far nodes
+// (800k bodies: walk 0.399 -> 0.392 ms; 16.8M: 7.87 -> 7.69 ms).
+__device__ __noinline__ void far_batch(const GNode* __restrict__ gnode, const uint32_t* ids,
+                                       float (&cacc)[kFarCoeffs], int lane, int cnt, float gcx,
+                                       float gcy, float lam, float eps2) {
     if (lane < cnt) {
-        const int j = nf_total - cnt + lane;
-        const float4 a = S.ent[cap - 1 - j][0];
-        const float4 b = S.ent[cap - 1 - j][1];
+        // (two 128-bit loads: with a 256-bit one in a called function ptxas 12.9 crashes)
+        const GNode* gp = &gnode[ids[lane]];
+        const float4 a = __ldg(&gp->mom), b = __ldg(&gp->tail);
         far_node_coeffs(cacc, __fsub_rn(gcx, a.x), __fsub_rn(gcy, a.y), a.z, a.w, b.x, b.y, lam,
                         eps2);
     }
@@ -127,7 +119,7 @@ constexpr int walk_min_blocks(int bpl) { return bpl >= 4 ? BH_WALK_MIN_BLOCKS_12
 // interactions; the stepping walk carries no counters (as a runtime switch
 // their four 64-bit sums held 8 registers through the whole traversal and
 // cost 5% at 800k and 16.8M bodies, 8% for 64-body groups).  Shared memory:
-// one GroupSmem<FAR> per warp, dynamic (the block shape is chosen at
+// one GroupSmem per warp, dynamic (the block shape is chosen at
 // launch).
 template <int BPL, int MP, bool PLUMMER, bool FAR, bool COUNT>
 __global__ void __launch_bounds__(walk_max_threads(BPL), walk_min_blocks(BPL))
@@ -137,10 +129,10 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                   const WalkParams P, uint32_t* __restrict__ err) {
     constexpr int NP = BPL / 2;  // packed pairs per lane (BPL >= 2)
     extern __shared__ __align__(16) unsigned char walk_smem[];
-    GroupSmem<FAR>* smem = reinterpret_cast<GroupSmem<FAR>*>(walk_smem);
+    GroupSmem* smem = reinterpret_cast<GroupSmem*>(walk_smem);
     if (step_failed(err)) return;  // the tree of this step was not built
     const int lane = threadIdx.x & 31;
-    GroupSmem<FAR>& S = smem[threadIdx.x >> 5];
+    GroupSmem& S = smem[threadIdx.x >> 5];
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t n = P.n, nm1 = n - 1;
@@ -339,89 +331,47 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             const uint32_t v = has ? S.stack[sp - k + lane] : 0u;
             sp -= k;
             __syncwarp();
-            bool emit_node = false, emit_range = false, push = false;
+            bool emit_node = false, emit_far = false, emit_range = false, push = false;
             uint32_t r0 = 0, r1 = 0;
-            float4 mom = make_float4(0.f, 0.f, 0.f, 0.f), sq = mom;
             if (has) {
                 if (v >= nm1) {
                     emit_range = (v - nm1) >= sys_lo && (v - nm1) < sys_hi;
                     r0 = v - nm1;
                     r1 = 1;
                 } else {
-                    // the whole 64-B record in one round trip
-                    const GNode* gp = &gnode[v];
-                    const float4 box = __ldg(&gp->box);
-                    const float4 m4 = __ldg(&gp->mom);
-                    const float4 q4 = __ldg(&gp->quad);
-                    const uint4 lk = __ldg(&gp->link);
-                    const uint32_t f = lk.z, e = lk.z + lk.w;
-                    if (e <= sys_lo || f >= sys_hi) {
-                        // another system's subtree: no interaction
-                    } else if (f < sys_lo || e > sys_hi) {
-                        push = true;  // spans several systems: always open
-                        r0 = lk.x;
-                        r1 = lk.y;
-                    } else if (group_accepts(box, m4.x, m4.y, glox, gloy, ghix, ghiy, th2)) {
+                    float4 box, tr;
+                    ldg_half(&gnode[v].box, box, tr);
+                    const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
+                    bool outside = false, spans = false;
+                    if (P.num_systems > 0) {
+                        const float4 tail = __ldg(&gnode[v].tail);
+                        const uint32_t f = __float_as_uint(tail.z), e = f + __float_as_uint(tail.w);
+                        outside = e <= sys_lo || f >= sys_hi;  // another system's subtree
+                        spans = f < sys_lo || e > sys_hi;      // of several systems: always open
+                    }
+                    if (outside) {
+                        // no interaction
+                    } else if (!spans && group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2)) {
+                        r0 = v;
                         emit_node = true;
-                        mom = m4;
-                        sq = q4;
-                    } else if (lk.w <= (uint32_t)P.leaf_size) {
+                        if (FAR && far_on) {
+                            // far from the group: to its local expansion
+                            const float rx = __fsub_rn(tr.x, gcx), ry = __fsub_rn(tr.y, gcy);
+                            const float R2 = __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry));
+                            emit_far = rg2 < __fmul_rn(P.far_alpha2, R2);
+                            emit_node = !emit_far;
+                        }
+                    } else if ((small & 255u) <= (uint32_t)P.leaf_size) {
+                        // (a node of several systems holds more bodies than that)
                         emit_range = true;
-                        r0 = lk.z;
-                        r1 = lk.w;
+                        r0 = link_gamma(link) + 1u - (small >> 8);
+                        r1 = small & 255u;
                     } else {
                         push = true;
-                        r0 = lk.x;
-                        r1 = lk.y;
+                        r0 = link_left(link, nm1);
+                        r1 = link_right(link, nm1);
                     }
                 }
-            }
-            // Far field: an accepted node far from the group goes to the far list.
-            bool emit_far = false;
-            if (far_on && emit_node) {
-                const float rx = __fsub_rn(mom.x, gcx), ry = __fsub_rn(mom.y, gcy);
-                const float R2 = __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry));
-                emit_far = rg2 < __fmul_rn(P.far_alpha2, R2);
-                emit_node = !emit_far;
-            }
-            if (FAR && far_on) {
-                const unsigned mf = __ballot_sync(FULL, emit_far);
-                if (emit_far) {
-                    const int q = GroupSmem<FAR>::kListCap - 1 - (nf + __popc(mf & lt));
-                    const bool quad = MP >= 2;
-                    S.ent[q][0] = make_float4(mom.x, mom.y, mom.z, quad ? sq.x : 0.f);
-                    S.ent[q][1] = make_float4(quad ? sq.y : 0.f, quad ? sq.z : 0.f, 0.f, 0.f);
-                }
-                nf += __popc(mf);
-            }
-            const unsigned mn = __ballot_sync(FULL, emit_node);
-            if (emit_node) {
-                const int p = nn + __popc(mn & lt);
-                S.ent[p][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
-                if (MP >= 2) {
-                    // -Q' = tr(S) I - 3S
-                    const float tr = sq.x + sq.z;
-                    const float nxx = tr - 3.0f * sq.x, nxy = -3.0f * sq.y, nyy = tr - 3.0f * sq.z;
-                    S.ent[p][1] = make_float4(mom.z, mom.z, nxx, nxx);
-                    S.ent[p][2] = make_float4(nxy, nxy, nyy, nyy);
-                } else {
-                    S.ent[p][1] = make_float4(mom.z, mom.z, 0.f, 0.f);
-                }
-            }
-            nn += __popc(mn);
-            {
-                // Append this step's body slots: exclusive scan of the counts.
-                const uint32_t c = emit_range ? r1 : 0u;
-                uint32_t incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                const uint32_t total = __shfl_sync(FULL, incl, 31);
-                const uint32_t at = (uint32_t)ns + incl - c;
-                for (uint32_t u = 0; u < c; ++u) S.slot[at + u] = r0 + u;
-                ns += (int)total;
             }
             const unsigned mp = __ballot_sync(FULL, push);
             const int npush = 2 * __popc(mp);
@@ -435,16 +385,54 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             } else if (lane == 0) {
                 atomicOr(err, kErrGroupStack);
             }
+            if (FAR) {
+                const unsigned mf = __ballot_sync(FULL, emit_far);
+                if (emit_far) S.far[nf + __popc(mf & lt)] = r0;
+                nf += __popc(mf);
+            }
+            const unsigned mn = __ballot_sync(FULL, emit_node);
+            if (emit_node) S.near[nn + __popc(mn & lt)] = r0;
+            nn += __popc(mn);
+            if (__any_sync(FULL, emit_range)) {
+                // Append this step's body slots: exclusive scan of the counts.
+                const uint32_t c = emit_range ? r1 : 0u;
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                const uint32_t total = __shfl_sync(FULL, incl, 31);
+                const uint32_t at = (uint32_t)ns + incl - c;
+                for (uint32_t u = 0; u < c; ++u) S.slot[at + u] = r0 + u;
+                ns += (int)total;
+            }
             if (counting) c_vis += (unsigned long long)k;
             __syncwarp();
             // Lists are evaluated when full, and whatever they hold once the
             // stack is empty; one call site each keeps the kernel's code
             // (and its instruction-cache footprint) small.
             const bool last = sp == 0;
-            if (nn >= 32 || (last && nn > 0)) {
-                eval_nodes(nn);
-                if (counting) c_node += (unsigned long long)nn * nvalid;
-                nn = 0;
+            while (nn >= 32 || (last && nn > 0)) {
+                const int cnt = nn < 32 ? nn : 32;
+                nn -= cnt;
+                if (lane < cnt) {
+                    float4 mom, tail;  // {com, mass, Sxx}, {Sxy, Syy}
+                    ldg_half(&gnode[S.near[nn + lane]].mom, mom, tail);
+                    S.ent[lane][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
+                    if (MP >= 2) {
+                        // -Q' = tr(S) I - 3S
+                        const float sxx = mom.w, sxy = tail.x, syy = tail.y, trS = sxx + syy;
+                        const float nxx = trS - 3.0f * sxx, nxy = -3.0f * sxy, nyy = trS - 3.0f * syy;
+                        S.ent[lane][1] = make_float4(mom.z, mom.z, nxx, nxx);
+                        S.ent[lane][2] = make_float4(nxy, nxy, nyy, nyy);
+                    } else {
+                        S.ent[lane][1] = make_float4(mom.z, mom.z, 0.f, 0.f);
+                    }
+                }
+                __syncwarp();
+                eval_nodes(cnt);
+                if (counting) c_node += (unsigned long long)cnt * nvalid;
                 __syncwarp();
             }
             if (ns >= 32 || (last && ns > 0)) {
@@ -455,9 +443,9 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             if constexpr (FAR) {
                 while (nf >= 32 || (last && nf > 0)) {
                     const int cnt = nf < 32 ? nf : 32;
-                    far_batch(S, cacc, lane, nf, cnt, gcx, gcy, lam, eps2);
-                    if (counting) c_far += (unsigned long long)cnt;
                     nf -= cnt;
+                    far_batch(gnode, S.far + nf, cacc, lane, cnt, gcx, gcy, lam, eps2);
+                    if (counting) c_far += (unsigned long long)cnt;
                     far_used = true;
                 }
             }
@@ -550,7 +538,7 @@ static int shape_index(int warps) { return warps == 2 ? 0 : (warps == 8 ? 2 : 1)
 
 template <int BPL, int MP, bool PL, bool FAR>
 static cudaError_t set_walk_attributes() {
-    const int smem = (int)(walk_max_threads(BPL) / 32 * sizeof(GroupSmem<FAR>));
+    const int smem = (int)(walk_max_threads(BPL) / 32 * sizeof(GroupSmem));
     cudaError_t e = cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -566,7 +554,7 @@ static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, cud
     static int blocks_per_sm[64][3] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    const size_t smem = (size_t)warps * sizeof(GroupSmem<FAR>);
+    const size_t smem = (size_t)warps * sizeof(GroupSmem);
     int& bps = blocks_per_sm[dev & 63][shape_index(warps)];
     if (bps == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(
