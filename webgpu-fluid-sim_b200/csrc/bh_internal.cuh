@@ -101,7 +101,7 @@ __device__ __forceinline__ bool group_accepts(const float4& box, float cx, float
     const float L = fmaxf(__fsub_rn(box.z, box.x), __fsub_rn(box.w, box.y));
     const float sx = fmaxf(__fsub_rn(box.x, ghix), __fsub_rn(glox, box.z));
     const float sy = fmaxf(__fsub_rn(box.y, ghiy), __fsub_rn(gloy, box.w));
-    return __fmul_rn(L, L) < __fmul_rn(th2, d2) && (sx > 0.0f || sy > 0.0f);
+    return (__fmul_rn(L, L) < __fmul_rn(th2, d2)) & (fmaxf(sx, sy) > 0.0f);  // no branch
 }
 
 // True when an earlier stage of this step left no valid input (its bounded

@@ -15,7 +15,8 @@
 // Derivatives of g (Faa di Bruno for g = h(|R|^2), h(u) = (u + eps^2)^-1/2):
 //     d^(a,b) g = s^(a+b+1) P_ab(rho),  s = (|R|^2 + eps^2)^-1/2,  rho = s R,
 //     P_ab = sum_{i<=a/2, j<=b/2} c(a,i) c(b,j) rho_x^(a-2i) rho_y^(b-2j) w(a+b-i-j),
-//     c(a,i) = a! / (i! (a-2i)! 2^i),  w(m) = (-1)^m (2m-1)!!.
+//     c(a,i) = a! / (i! (a-2i)! 2^i),  w(m) = (-1)^m (2m-1)!!
+// (evaluated order by order with a recurrence, far_next).
 // With the length scale lambda = r_g and t = lambda s (< alpha for a far node)
 // the scaled coefficients of orders 1..4 (kFarCoeffs of them) are
 //     C_ab = lambda^(a+b) d^(a,b) Phi(x_g)
@@ -33,6 +34,7 @@
 #pragma once
 
 #include "bh_internal.cuh"
+#include "packed.cuh"
 
 namespace bh {
 
@@ -42,85 +44,76 @@ constexpr int kFarCoeffs = 14;  // potential coefficients of orders 1..4
 __host__ __device__ constexpr int far_idx(int a, int b) {
     return (a + b - 1) * (a + b + 2) / 2 + b;
 }
-__host__ __device__ constexpr float far_c(int a, int i) {
-    // a! / (i! (a - 2i)! 2^i)
-    float num = 1.f;
-    for (int k = 2; k <= a; ++k) num *= (float)k;
-    float den = 1.f;
-    for (int k = 2; k <= i; ++k) den *= (float)k;
-    for (int k = 2; k <= a - 2 * i; ++k) den *= (float)k;
-    for (int k = 0; k < i; ++k) den *= 2.f;
-    return num / den;
-}
-__host__ __device__ constexpr float far_w(int m) {
-    // (-1)^m (2m - 1)!!
-    float v = 1.f;
-    for (int k = 1; k <= m; ++k) v *= -(float)(2 * k - 1);
-    return v;
-}
-
-// P_ab(rho) from the powers ex[k] = rho_x^k, ey[k] = rho_y^k (k <= 6).
-template <int A, int B>
-__device__ __forceinline__ float far_poly(const float (&ex)[7], const float (&ey)[7]) {
-    float acc = 0.f;
+// P_ab of the next order from the two orders below it (prev: order N - 1 by b,
+// last: order N), for two nodes at once.  From u dg/dx = -x g, u = |R|^2 + eps^2,
+// differentiated a - 1 times in x and b times in y and scaled as above:
+//     P_ab = -[ (2a-1) rho_x P_(a-1)b + (a-1)^2 P_(a-2)b
+//               + 2b rho_y P_a(b-1) + b(b-1) P_a(b-2) ]        (a >= 1)
+// and the same with x and y exchanged for a = 0.  Two to four fused
+// multiply-adds per value, half of what the closed sums take.
+template <int N>
+__device__ __forceinline__ void far_next(f2x (&next)[N + 2], const f2x (&last)[N + 1],
+                                         const f2x* prev, f2x rhx, f2x rhy) {
+    auto c2 = [](float v) { return pk(v, v); };
 #pragma unroll
-    for (int i = 0; 2 * i <= A; ++i)
-#pragma unroll
-        for (int j = 0; 2 * j <= B; ++j)
-            acc = __fmaf_rn(far_c(A, i) * far_c(B, j) * far_w(A + B - i - j),
-                            __fmul_rn(ex[A - 2 * i], ey[B - 2 * j]), acc);
-    return acc;
-}
-
-// One coefficient C_ab of one node, added to acc[far_idx(a, b)].
-template <int A, int B>
-__device__ __forceinline__ void far_term(float* acc, const float (&ex)[7], const float (&ey)[7],
-                                         float m, float sxx, float sxy, float syy,
-                                         const float (&st)[5]) {
-    const float quad = __fmaf_rn(sxx, far_poly<A + 2, B>(ex, ey),
-                        __fmaf_rn(2.f * sxy, far_poly<A + 1, B + 1>(ex, ey),
-                                  __fmul_rn(syy, far_poly<A, B + 2>(ex, ey))));
-    const float v = __fmaf_rn(m, far_poly<A, B>(ex, ey), __fmul_rn(0.5f, quad));
-    acc[far_idx(A, B)] = __fmaf_rn(-st[A + B], v, acc[far_idx(A, B)]);
-}
-
-// Add one node's scaled local coefficients (about x_g, length scale lambda)
-// to acc[kFarCoeffs].  R = x_g - c.
-__device__ __forceinline__ void far_node_coeffs(float (&acc)[kFarCoeffs], float rx, float ry, float m, float sxx,
-                                                float sxy, float syy, float lambda, float eps2) {
-    const float u = __fadd_rn(__fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry)), eps2);
-    const float s = __frsqrt_rn(u);
-    const float s2 = __fmul_rn(s, s);
-    float ex[7], ey[7];
-    ex[0] = 1.f;
-    ey[0] = 1.f;
-    ex[1] = __fmul_rn(rx, s);
-    ey[1] = __fmul_rn(ry, s);
-#pragma unroll
-    for (int k = 2; k < 7; ++k) {
-        ex[k] = __fmul_rn(ex[k - 1], ex[1]);
-        ey[k] = __fmul_rn(ey[k - 1], ey[1]);
+    for (int b = 0; b <= N; ++b) {
+        const int a = N + 1 - b;
+        f2x v = mul2(mul2(rhx, last[b]), c2(-(float)(2 * a - 1)));  // P_(a-1)b
+        if (a >= 2 && N >= 1) v = fma2(prev[b], c2(-(float)((a - 1) * (a - 1))), v);      // P_(a-2)b
+        if (b >= 1) v = fma2(mul2(rhy, last[b - 1]), c2(-(float)(2 * b)), v);             // P_a(b-1)
+        if (b >= 2) v = fma2(prev[b - 2], c2(-(float)(b * (b - 1))), v);                  // P_a(b-2)
+        next[b] = v;
     }
-    const float t = __fmul_rn(lambda, s);
-    float st[5];
-    st[0] = s;
+    f2x v = mul2(mul2(rhy, last[N]), c2(-(float)(2 * N + 1)));
+    if (N >= 1) v = fma2(prev[N - 1], c2(-(float)(N * N)), v);
+    next[N + 1] = v;
+}
+
+// Add the coefficients of order N of two nodes to acc: st = s t^N, p / q = P
+// of order N / N + 2, hxx = S'xx / 2, qxy = S'xy, hyy = S'yy / 2.
+template <int N>
+__device__ __forceinline__ void far_order(float (&acc)[kFarCoeffs], const f2x (&p)[N + 1],
+                                          const f2x (&q)[N + 3], f2x m, f2x hxx, f2x qxy, f2x hyy,
+                                          f2x st) {
 #pragma unroll
-    for (int k = 1; k < 5; ++k) st[k] = __fmul_rn(st[k - 1], t);
-    const float qxx = __fmul_rn(s2, sxx), qxy = __fmul_rn(s2, sxy), qyy = __fmul_rn(s2, syy);
-    far_term<1, 0>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<0, 1>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<2, 0>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<1, 1>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<0, 2>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<3, 0>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<2, 1>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<1, 2>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<0, 3>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<4, 0>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<3, 1>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<2, 2>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<1, 3>(acc, ex, ey, m, qxx, qxy, qyy, st);
-    far_term<0, 4>(acc, ex, ey, m, qxx, qxy, qyy, st);
+    for (int b = 0; b <= N; ++b) {
+        const f2x v = fma2(m, p[b], fma2(hxx, q[b], fma2(qxy, q[b + 1], mul2(hyy, q[b + 2]))));
+        acc[far_idx(N - b, b)] -= sum_halves(mul2(st, v));
+    }
+}
+
+// Add the scaled local coefficients (about x_g, length scale lambda) of two
+// nodes, one per half, to acc[kFarCoeffs].  R = x_g - c.  A half with m = S = 0
+// (and any finite R) adds nothing.
+__device__ __forceinline__ void far_node_coeffs(float (&acc)[kFarCoeffs], f2x rx, f2x ry, f2x m,
+                                                f2x sxx, f2x sxy, f2x syy, float lambda,
+                                                float eps2) {
+    const f2x u = fma2(rx, rx, fma2(ry, ry, pk(eps2, eps2)));
+    f2x s = rsqrt2(u);
+    // One Newton step: s is good to half a unit in the last place or so.  (An
+    // overflowed u leaves s = 0 and adds nothing, hence the finite bound.)
+    const f2x half = pk(0.5f, 0.5f);
+    float u0, u1;
+    upk(u, u0, u1);
+    const f2x nu = pk(-fminf(u0, 3.0e38f), -fminf(u1, 3.0e38f));
+    s = fma2(mul2(s, half), fma2(mul2(nu, s), s, pk(1.f, 1.f)), s);
+    const f2x rhx = mul2(rx, s), rhy = mul2(ry, s), s2 = mul2(s, s), t = mul2(pk(lambda, lambda), s);
+    const f2x hxx = mul2(mul2(s2, sxx), half), qxy = mul2(s2, sxy), hyy = mul2(mul2(s2, syy), half);
+    f2x p0[1] = {pk(1.f, 1.f)}, p1[2], p2[3], p3[4], p4[5], p5[6], p6[7];
+    far_next<0>(p1, p0, nullptr, rhx, rhy);
+    far_next<1>(p2, p1, p0, rhx, rhy);
+    far_next<2>(p3, p2, p1, rhx, rhy);
+    f2x st = mul2(s, t);
+    far_order<1>(acc, p1, p3, m, hxx, qxy, hyy, st);
+    far_next<3>(p4, p3, p2, rhx, rhy);
+    st = mul2(st, t);
+    far_order<2>(acc, p2, p4, m, hxx, qxy, hyy, st);
+    far_next<4>(p5, p4, p3, rhx, rhy);
+    st = mul2(st, t);
+    far_order<3>(acc, p3, p5, m, hxx, qxy, hyy, st);
+    far_next<5>(p6, p5, p4, rhx, rhy);
+    st = mul2(st, t);
+    far_order<4>(acc, p4, p6, m, hxx, qxy, hyy, st);
 }
 
 // Force of the local expansion at offset d = (x - x_g) / lambda:

@@ -27,32 +27,49 @@
 // Leaves, and opened nodes of <= leaf_size bodies, are summed body by body.
 //
 // Traversal: a per-warp stack in shared memory.  Every step each lane takes
-// one of the top 32 stack entries, loads its whole 64-B record in one round
-// trip, evaluates it, and the warp compacts the outcomes (ballots and a
-// warp scan) into a node list, a body-slot list and the stack.  Lists are
-// evaluated when they hold >= 32 entries: every lane runs every entry for its
-// BPL bodies (shared-memory broadcasts, no divergence); body records are
-// first loaded 32 at a time by the 32 lanes in parallel.
+// one of the top 32 stack entries, loads the half record the decision needs
+// with one 256-bit load, decides without branching (a step is a chain of
+// dependent instructions), and the warp compacts the outcomes by ballots into
+// a node list, a far list, a list of body ranges and the stack.  A list is
+// evaluated when it holds 32 entries (far: 64): nodes and bodies are staged in
+// shared memory 32 at a time by the 32 lanes in parallel, then every lane
+// runs every entry for its BPL bodies (shared-memory broadcasts, no
+// divergence).
 // Above kWalkDfsAt entries the warp pops one node per step (plain DFS), which
 // keeps the stack below kWalkStack for any tree of depth <= 96; a push that
 // would not fit raises kErrGroupStack instead of writing out of bounds.
-// Groups are taken from an atomic counter (the walk is persistent).
+// Groups are taken from an atomic counter (the walk is persistent).  (Taking
+// the next group early, to hide that round trip, lengthened the drain: 800k
+// walk 359 -> 395 us.  Sharing one traversal among the groups of a larger
+// subtree, through lists in global memory, was twice as slow: the groups'
+// union of nodes is 1.7 times one group's, and a list step of one warp takes
+// as long as a traversal step here.)
 //
-// Packed arithmetic: with BPL >= 2 each lane evaluates its bodies in pairs
-// with the sm_100 packed FP32 instructions (add/sub/mul/fma .rn.f32x2), one
-// instruction for both bodies.  Node-list entries are stored in shared memory
-// with every value duplicated ({cx,cx,cy,cy}, ...), so a 128-bit shared load
-// yields ready operand pairs, and with the quadrupole negated so every
-// accumulation is a plain fused multiply-add.  With eps^2 > 0 a body's own
-// leaf adds exactly zero (r = 0), so no self test is needed.
+// Packed arithmetic: each lane evaluates two interactions per instruction with
+// the sm_100 packed FP32 instructions (add/sub/mul/fma .rn.f32x2).  Sub-slots
+// (32 bodies, one per lane) go two to a pair; staged entries then hold every
+// value twice ({cx,cx,cy,cy}, ...), so a 128-bit shared load yields ready
+// operand pairs.  An odd sub-slot takes two list entries per instruction
+// instead, from a second staged copy ({cx_j,cx_j+1, ...}): groups of 65..96
+// bodies cost 1.5 pairs an entry, not 2 (15% fewer evaluations at 800k).  The
+// quadrupole is stored negated so every accumulation is a plain fused
+// multiply-add.  With eps^2 > 0 a body's own leaf adds exactly zero (r = 0),
+// so no self test is needed.
 //
 // Far field (far_alpha > 0, extension): an accepted node whose COM lies far
 // from the group compared with the group's size (r_g < far_alpha R, r_g the
 // group box's half-diagonal, R the distance from the box centre to the COM)
-// is not evaluated body by body.  Lanes turn 32 such nodes at a time into
-// the coefficients of a local expansion about the box centre, each lane
-// summing its own in registers; at the end of the group the lanes' sums are
-// reduced and every body evaluates the expansion once (far_field.cuh).
+// is not evaluated body by body.  Lanes turn 64 such nodes at a time, two
+// each, into the coefficients of a local expansion about the box centre, each
+// lane summing its own; at the end of the group the lanes' sums are reduced
+// and every body evaluates the expansion once (far_field.cuh).
+//
+// What bounds it (B200, 800k colliding disks, 128-body groups, leaf 4): 189M
+// warp instructions at 62% of the issue slots, 24 warps per SM, FMA pipe 47%;
+// the last 14% of the launch is the drain of the last groups.  Walk stage
+// before the branch-free step, id lists, packed far batches and passes over
+// one loop -> now: 800k 389 -> 305 us, 16.8M 7.61 -> 5.80 ms, 64-body groups
+// (ensemble of 64 systems, 1.2M bodies) 584 -> 438 us.
 #include "bh_internal.cuh"
 #include "far_field.cuh"
 #include "packed.cuh"
@@ -63,37 +80,62 @@ namespace bh {
 // more warps reach the one-node-per-step depth guard.
 constexpr int kWalkStack = 320;
 constexpr int kWalkDfsAt = kWalkStack - 128;  // >= 32 + 96 below the capacity
+// Where an empty staged entry lies: massless, and far from any body.
+constexpr float kFarAway = 1.0e18f;
 
-constexpr int kSlotList = 32 + 32 * kGroupMaxLeaf;  // body slots: < 32 kept + one step's adds
-// A warp's shared memory.  The lists hold node ids and slots: a step adds at
-// most 32 ids to fewer than 32 kept ones.  Nodes and bodies are staged 32 at a
-// time for their evaluation.
+// A warp's shared memory.  The lists hold node ids and body ranges: a step adds
+// at most 32 to fewer than 32 kept ones (far: 64).  32 ranges at a time are
+// expanded to slots; nodes and bodies are staged 32 at a time for their
+// evaluation.
 struct GroupSmem {
     uint32_t stack[kWalkStack];
-    // staged node j: ent[j][0] = {cx, cx, cy, cy}, ent[j][1] = {m, m, -Q'xx, -Q'xx},
-    //                ent[j][2] = {-Q'xy, -Q'xy, -Q'yy, -Q'yy}
-    float4 ent[32][3];
-    float4 body[32][2];        // staged leaf records as pairs {x,x,y,y}, {m,m,0,0}
+    // staged nodes, as operand pairs: ent[j][0] = {cx, cx, cy, cy},
+    // ent[j][1] = {m, m, -Q'xx, -Q'xx}, ent[j][2] = {-Q'xy, -Q'xy, -Q'yy, -Q'yy};
+    // ent2: the same with nodes 2j and 2j + 1 in the two places of each value
+    // (never staged at the same time as the leaf records: every bit of shared
+    // memory saved is L1 for the node records)
+    struct Nodes {
+        float4 ent[32][3];
+        float4 ent2[16][3];
+    };
+    // staged leaf records: {x, x, y, y}, {m, m, slot bits, slot bits}; body2: two per entry
+    struct Bodies {
+        float4 body[32][2];
+        float4 body2[16][2];
+    };
+    union {
+        Nodes nodes;
+        Bodies bodies;
+    };
     uint32_t near[64];         // nodes to evaluate at each body
-    uint32_t far[64];          // nodes for the group's local expansion
-    uint32_t slot[kSlotList];  // sorted slots of bodies to sum one by one
+    uint32_t far[96];          // nodes for the group's local expansion (evaluated 64 at a time)
+    uint32_t first[64];        // ranges of bodies to sum one by one: first slot,
+    unsigned char count[64];   // and how many
+    uint32_t slot[32 * kGroupMaxLeaf];
 };
 
-// Far list: one node per lane (lane < cnt) added to the lane's local-expansion
-// sums.  Not inlined: the coefficient arithmetic is the walk's register peak,
-// and as a call (the caller's live values saved around it, the sums in a 56-B
-// stack frame) the 128-body far-field walk fits 6 blocks per SM in 80
-// registers instead of 5 in 96.  A call costs little once per 32 far nodes
-// (800k bodies: walk 0.399 -> 0.392 ms; 16.8M: 7.87 -> 7.69 ms).
+// Far list: two nodes per lane (ids[lane], ids[32 + lane], below cnt <= 64)
+// added to the lane's local-expansion sums, both in one packed instruction
+// stream.  Not inlined: the coefficient arithmetic is the walk's register peak
+// (inlined: 800k 316 against 305 us, 16.8M 6.03 / 5.80 ms; 32 nodes a batch
+// instead of 64: 317 us, 6.13 ms).
 __device__ __noinline__ void far_batch(const GNode* __restrict__ gnode, const uint32_t* ids,
                                        float (&cacc)[kFarCoeffs], int lane, int cnt, float gcx,
-                                       float gcy, float lam, float eps2) {
+                                       float gcy, float rg2, float eps2) {
     if (lane < cnt) {
+        const float lam = __fsqrt_rn(rg2);  // the expansion's length scale
         // (two 128-bit loads: with a 256-bit one in a called function ptxas 12.9 crashes)
         const GNode* gp = &gnode[ids[lane]];
         const float4 a = __ldg(&gp->mom), b = __ldg(&gp->tail);
-        far_node_coeffs(cacc, __fsub_rn(gcx, a.x), __fsub_rn(gcy, a.y), a.z, a.w, b.x, b.y, lam,
-                        eps2);
+        float4 c = make_float4(a.x, a.y, 0.f, 0.f), d = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane + 32 < cnt) {
+            const GNode* gq = &gnode[ids[lane + 32]];
+            c = __ldg(&gq->mom);
+            d = __ldg(&gq->tail);
+        }
+        far_node_coeffs(cacc, pk(__fsub_rn(gcx, a.x), __fsub_rn(gcx, c.x)),
+                        pk(__fsub_rn(gcy, a.y), __fsub_rn(gcy, c.y)), pk(a.z, c.z), pk(a.w, c.w),
+                        pk(b.x, d.x), pk(b.y, d.y), lam, eps2);
     }
     __syncwarp();
 }
@@ -101,15 +143,14 @@ __device__ __noinline__ void far_batch(const GNode* __restrict__ gnode, const ui
 // Register budget: launch bounds for blocks of up to 256 threads with 3
 // resident per SM for groups of <= 64 bodies (at most 85 registers, the
 // budget of 6 resident 128-thread blocks); for 128-body groups blocks of up
-// to 128 threads with 6 resident (at most 85: 80 for the far-field walk with
-// its coefficient routine called, not inlined).  The bound does not depend
-// on the block shape chosen at launch (walk_block: 64, 128 or, for groups of
-// <= 64 bodies, 256 threads), so the shape leaves the warps resident per SM
-// unchanged.  (An explicit register cap of 72 in place of these bounds gave
-// a 65-register build of the 64-body walk that ran 12% slower.)
+// to 128 threads with 5 resident (96 registers, no spills; with 6 the
+// far-field walk spills: 800k 313 against 305 us, 16.8M 5.85 / 5.80 ms; 7 and
+// 8 were slower still).  The bound does not depend on the block shape chosen
+// at launch (walk_block: 64, 128 or, for groups of <= 64 bodies, 256
+// threads), so the shape leaves the warps resident per SM unchanged.
 constexpr int walk_max_threads(int bpl) { return bpl >= 4 ? 128 : 256; }
 #ifndef BH_WALK_MIN_BLOCKS_128
-#define BH_WALK_MIN_BLOCKS_128 6
+#define BH_WALK_MIN_BLOCKS_128 5
 #endif
 constexpr int walk_min_blocks(int bpl) { return bpl >= 4 ? BH_WALK_MIN_BLOCKS_128 : 3; }
 
@@ -127,7 +168,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                   const uint2* __restrict__ groups, const uint32_t* __restrict__ ids,
                   float2* __restrict__ pos, float2* __restrict__ vel, float2* __restrict__ acc,
                   const WalkParams P, uint32_t* __restrict__ err) {
-    constexpr int NP = BPL / 2;  // packed pairs per lane (BPL >= 2)
+    constexpr int NP = (BPL + 1) / 2;  // packed pairs per lane
     extern __shared__ __align__(16) unsigned char walk_smem[];
     GroupSmem* smem = reinterpret_cast<GroupSmem*>(walk_smem);
     if (step_failed(err)) return;  // the tree of this step was not built
@@ -194,131 +235,157 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
         const float gcy = __fmul_rn(0.5f, __fadd_rn(gloy, ghiy));
         const float ghx = __fsub_rn(ghix, glox), ghy = __fsub_rn(ghiy, gloy);
         const float rg2 = __fmul_rn(0.25f, __fadd_rn(__fmul_rn(ghx, ghx), __fmul_rn(ghy, ghy)));
-        const bool far_on = FAR && PLUMMER && P.far_alpha2 > 0.0f && rg2 > 0.0f;
-        const float lam = far_on ? __fsqrt_rn(rg2) : 1.0f;
+        // (infinite: no node is far)
+        const float far_rg2 = FAR && PLUMMER && P.far_alpha2 > 0.0f && rg2 > 0.0f ? rg2 : INFINITY;
         bool far_used = false;
         float cacc[kFarCoeffs];  // this lane's local-expansion sums
 #pragma unroll
         for (int k = 0; k < kFarCoeffs; ++k) cacc[k] = 0.0f;
-        // Accumulators: packed pairs (BPL >= 2) or scalars (BPL == 1).
-        f2x X[NP > 0 ? NP : 1], Y[NP > 0 ? NP : 1], AX[NP > 0 ? NP : 1], AY[NP > 0 ? NP : 1];
-        float ax1 = 0.f, ay1 = 0.f;
+        // The lane's bodies in packed pairs: pair q holds sub-slots 2q and 2q+1.
+        // With an odd number of sub-slots in use the last one is held twice in
+        // the last pair, whose halves take alternate list entries.
+        const bool odd = kmax & 1;
+        const int full = kmax >> 1;  // pairs of two sub-slots
+        f2x X[NP], Y[NP], AX[NP], AY[NP];
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
-            X[q] = pk(bx[2 * q], bx[2 * q + 1]);
-            Y[q] = pk(by[2 * q], by[2 * q + 1]);
+            X[q] = pk(bx[2 * q], bx[BPL > 1 ? 2 * q + 1 : 0]);
+            Y[q] = pk(by[2 * q], by[BPL > 1 ? 2 * q + 1 : 0]);
             AX[q] = pk(0.f, 0.f);
             AY[q] = pk(0.f, 0.f);
+        }
+        float odd_m = bm[0];
+        if (BPL > 1 && odd) {
+            constexpr int k2 = BPL > 2 ? 2 : 0;
+            const bool third = kmax == 3;
+            const float ox = third ? bx[k2] : bx[0], oy = third ? by[k2] : by[0];
+            X[NP - 1] = pk(ox, ox);
+            Y[NP - 1] = pk(oy, oy);
+            odd_m = third ? bm[k2] : bm[0];
         }
         const f2x E2 = pk(eps2, eps2);
         const f2x M25 = pk(-2.5f, -2.5f);
 
-        auto soft_pair = [&](int q, float m2) -> f2x {
+        // The lists are evaluated in passes, one per pair in use: the pairs of
+        // two sub-slots over ent / body, the odd one over ent2 / body2 (half as
+        // many entries).  All passes run the same loop: the kernel's code has
+        // to stay small (with a loop for each case the instruction cache
+        // thrashed: 4.1 of 9.7 stall cycles an issue, 800k walk 378 us).
+        const int passes = full + (odd ? 1 : 0);
+        // squared softening of a pair of interactions
+        auto soft = [&](f2x M, float ma, float mb) -> f2x {
             if (PLUMMER) return E2;
-            return pk(ecoef * fmaxf(bm[2 * q], m2), ecoef * fmaxf(bm[2 * q + 1], m2));
+            float lo, hi;
+            upk(M, lo, hi);
+            return pk(ecoef * fmaxf(ma, lo), ecoef * fmaxf(mb, hi));
         };
-
-        // Node list: multipole interactions.
-        auto eval_nodes = [&](int cnt) {
-#pragma unroll 4  // four independent entries in flight per lane (measured best)
-            for (int j = 0; j < cnt; ++j) {
-                const float4 e0 = S.ent[j][0], e1 = S.ent[j][1];
-                float4 e2 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (MP >= 2) e2 = S.ent[j][2];
-                if (NP > 0) {
-                    const f2x CX = ld_pair(e0, 0), CY = ld_pair(e0, 1), M = ld_pair(e1, 0);
-#pragma unroll
-                    for (int q = 0; q < NP; ++q) {
-                        if (2 * q >= kmax) break;
-                        const f2x rx = sub2(CX, X[q]), ry = sub2(CY, Y[q]);
-                        const f2x r2 = fma2(rx, rx, fma2(ry, ry, soft_pair(q, e1.x)));
-                        const f2x inv = rsqrt2(r2);
-                        const f2x inv2 = mul2(inv, inv);
-                        const f2x inv3 = mul2(inv, inv2);
-                        if (MP >= 2) {
-                            const f2x NQXX = ld_pair(e1, 1), NQXY = ld_pair(e2, 0), NQYY = ld_pair(e2, 1);
-                            const f2x nqrx = fma2(NQXX, rx, mul2(NQXY, ry));  // -(Q'r)_x
-                            const f2x nqry = fma2(NQXY, rx, mul2(NQYY, ry));  // -(Q'r)_y
-                            const f2x nrqr = fma2(rx, nqrx, mul2(ry, nqry)); // -r.Q'r
-                            const f2x inv5 = mul2(inv3, inv2);
-                            // f = m / |r|^3 + 5/2 r.Q'r / |r|^7
-                            const f2x f = fma2(mul2(nrqr, M25), mul2(inv5, inv2), mul2(M, inv3));
-                            AX[q] = fma2(nqrx, inv5, fma2(f, rx, AX[q]));
-                            AY[q] = fma2(nqry, inv5, fma2(f, ry, AY[q]));
-                        } else {
-                            const f2x mi3 = mul2(M, inv3);
-                            AX[q] = fma2(mi3, rx, AX[q]);
-                            AY[q] = fma2(mi3, ry, AY[q]);
-                        }
-                    }
+        auto for_passes = [&](auto&& body) {
+#pragma unroll 1
+            for (int ps = 0; ps < passes; ++ps) {
+                const bool is_odd = ps == full;
+                const bool lastp = NP > 1 && (ps == NP - 1 || is_odd);  // which register pair
+                const f2x x = lastp ? X[NP - 1] : X[0], y = lastp ? Y[NP - 1] : Y[0];
+                f2x ax2 = lastp ? AX[NP - 1] : AX[0], ay2 = lastp ? AY[NP - 1] : AY[0];
+                // masses and slots of the two bodies (softening by mass, self test)
+                const float ma = is_odd ? odd_m : (lastp ? bm[BPL > 2 ? 2 : 0] : bm[0]);
+                const float mb = is_odd ? odd_m : (lastp ? bm[BPL > 2 ? 3 : 0] : bm[BPL > 1 ? 1 : 0]);
+                const uint32_t sa = base + (uint32_t)lane + (is_odd ? 32u * (uint32_t)(kmax - 1) : 64u * (uint32_t)ps);
+                const uint32_t sb = is_odd ? sa : sa + 32u;
+                body(is_odd, x, y, ax2, ay2, ma, mb, sa, sb);
+                if (lastp) {
+                    AX[NP - 1] = ax2;
+                    AY[NP - 1] = ay2;
                 } else {
-                    const float rx = e0.x - bx[0], ry = e0.z - by[0];
-                    const float es = PLUMMER ? eps2 : ecoef * fmaxf(bm[0], e1.x);
-                    const float inv = rsqrt_ftz(fmaf(rx, rx, fmaf(ry, ry, es)));
-                    const float inv2 = inv * inv, inv3 = inv * inv2;
-                    const float mi3 = e1.x * inv3;
-                    if (MP >= 2) {
-                        const float nqrx = fmaf(e1.z, rx, e2.x * ry);
-                        const float nqry = fmaf(e2.x, rx, e2.z * ry);
-                        const float nrqr = fmaf(rx, nqrx, ry * nqry);
-                        const float inv5 = inv3 * inv2;
-                        const float f = fmaf(-2.5f * nrqr, inv5 * inv2, mi3);
-                        ax1 = fmaf(nqrx, inv5, fmaf(f, rx, ax1));
-                        ay1 = fmaf(nqry, inv5, fmaf(f, ry, ay1));
-                    } else {
-                        ax1 = fmaf(mi3, rx, ax1);
-                        ay1 = fmaf(mi3, ry, ay1);
-                    }
+                    AX[0] = ax2;
+                    AY[0] = ay2;
                 }
             }
         };
-        // Body list: point masses.  32 leaf records at a time are loaded by the
-        // 32 lanes in parallel into shared memory, then every lane sums them.
-        auto eval_bodies = [&](int cnt) {
-            for (int c0 = 0; c0 < cnt; c0 += 32) {
-                const int mcnt = (cnt - c0) < 32 ? (cnt - c0) : 32;
-                __syncwarp();
-                if (lane < mcnt) {
-                    const float4 o = __ldg(&node4[nm1 + S.slot[c0 + lane]]);
-                    S.body[lane][0] = make_float4(o.x, o.x, o.y, o.y);
-                    S.body[lane][1] = make_float4(o.z, o.z, 0.f, 0.f);
-                }
-                __syncwarp();
-                for (int j = 0; j < mcnt; ++j) {
-                    const float4 p0 = S.body[j][0], p1 = S.body[j][1];
-                    const uint32_t s = self_test ? S.slot[c0 + j] : 0u;
-                    if (NP > 0) {
-                        const f2x OX = ld_pair(p0, 0), OY = ld_pair(p0, 1), OM = ld_pair(p1, 0);
-#pragma unroll
-                        for (int q = 0; q < NP; ++q) {
-                            if (2 * q >= kmax) break;
-                            const f2x rx = sub2(OX, X[q]), ry = sub2(OY, Y[q]);
-                            const f2x r2 = fma2(rx, rx, fma2(ry, ry, soft_pair(q, p1.x)));
-                            const f2x inv = rsqrt2(r2);
-                            f2x f = mul2(OM, mul2(inv, mul2(inv, inv)));
-                            if (self_test) {
-                                const uint32_t s0 = base + (uint32_t)(2 * q) * 32u + (uint32_t)lane;
-                                float f0, f1;
-                                upk(f, f0, f1);
-                                f = pk(s == s0 ? 0.0f : f0, s == s0 + 32u ? 0.0f : f1);
-                            }
-                            AX[q] = fma2(f, rx, AX[q]);
-                            AY[q] = fma2(f, ry, AY[q]);
-                        }
+        // The staged nodes: multipole interactions.
+        auto eval_nodes = [&](int cnt) {
+            for_passes([&](bool is_odd, f2x x, f2x y, f2x& ax2, f2x& ay2, float ma, float mb, uint32_t, uint32_t) {
+                const float4(*e)[3] = is_odd ? S.nodes.ent2 : S.nodes.ent;
+                const int m = is_odd ? (cnt + 1) >> 1 : cnt;
+#pragma unroll 4  // four independent entries in flight per lane (measured best)
+                for (int j = 0; j < m; ++j) {
+                    const float4 e0 = e[j][0], e1 = e[j][1];
+                    const f2x M = ld_pair(e1, 0);
+                    const f2x rx = sub2(ld_pair(e0, 0), x), ry = sub2(ld_pair(e0, 1), y);
+                    const f2x r2 = fma2(rx, rx, fma2(ry, ry, soft(M, ma, mb)));
+                    const f2x inv = rsqrt2(r2);
+                    const f2x inv2 = mul2(inv, inv);
+                    const f2x inv3 = mul2(inv, inv2);
+                    if (MP >= 2) {
+                        const float4 e2 = e[j][2];
+                        const f2x NQXX = ld_pair(e1, 1), NQXY = ld_pair(e2, 0), NQYY = ld_pair(e2, 1);
+                        const f2x nqrx = fma2(NQXX, rx, mul2(NQXY, ry));  // -(Q'r)_x
+                        const f2x nqry = fma2(NQXY, rx, mul2(NQYY, ry));  // -(Q'r)_y
+                        const f2x nrqr = fma2(rx, nqrx, mul2(ry, nqry));  // -r.Q'r
+                        const f2x inv5 = mul2(inv3, inv2);
+                        // f = m / |r|^3 + 5/2 r.Q'r / |r|^7
+                        const f2x f = fma2(mul2(nrqr, M25), mul2(inv5, inv2), mul2(M, inv3));
+                        ax2 = fma2(nqrx, inv5, fma2(f, rx, ax2));
+                        ay2 = fma2(nqry, inv5, fma2(f, ry, ay2));
                     } else {
-                        const float rx = p0.x - bx[0], ry = p0.z - by[0];
-                        const float es = PLUMMER ? eps2 : ecoef * fmaxf(bm[0], p1.x);
-                        const float inv = rsqrt_ftz(fmaf(rx, rx, fmaf(ry, ry, es)));
-                        float f = p1.x * (inv * inv * inv);
-                        if (self_test) f = (s == base + (uint32_t)lane) ? 0.0f : f;
-                        ax1 = fmaf(f, rx, ax1);
-                        ay1 = fmaf(f, ry, ay1);
+                        const f2x mi3 = mul2(M, inv3);
+                        ax2 = fma2(mi3, rx, ax2);
+                        ay2 = fma2(mi3, ry, ay2);
                     }
                 }
+            });
+        };
+        // The bodies listed in S.slot: point masses.  32 leaf records at a time
+        // are loaded by the 32 lanes in parallel into shared memory.
+        auto eval_bodies = [&](int total) {
+            for (int c0 = 0; c0 < total; c0 += 32) {
+                const int cnt = (total - c0) < 32 ? (total - c0) : 32;
+                __syncwarp();
+                {
+                    float4 o = make_float4(kFarAway, kFarAway, 0.f, 0.f);
+                    float sl = __uint_as_float(kSentinel);
+                    if (lane < cnt) {
+                        const uint32_t slot = S.slot[c0 + lane];
+                        o = __ldg(&node4[nm1 + slot]);
+                        sl = __uint_as_float(slot);
+                    }
+                    if (full > 0) {
+                        S.bodies.body[lane][0] = make_float4(o.x, o.x, o.y, o.y);
+                        S.bodies.body[lane][1] = make_float4(o.z, o.z, sl, sl);
+                    }
+                    if (odd) {
+                        float* const d = reinterpret_cast<float*>(&S.bodies.body2[lane >> 1][0]) + (lane & 1);
+                        d[0] = o.x;
+                        d[2] = o.y;
+                        d[4] = o.z;
+                        d[6] = sl;
+                    }
+                }
+                __syncwarp();
+                for_passes([&](bool is_odd, f2x x, f2x y, f2x& ax2, f2x& ay2, float ma, float mb, uint32_t sa, uint32_t sb) {
+                    const float4(*e)[2] = is_odd ? S.bodies.body2 : S.bodies.body;
+                    const int m = is_odd ? (cnt + 1) >> 1 : cnt;
+#pragma unroll 4
+                    for (int j = 0; j < m; ++j) {
+                        const float4 p0 = e[j][0], p1 = e[j][1];
+                        const f2x OM = ld_pair(p1, 0);
+                        const f2x rx = sub2(ld_pair(p0, 0), x), ry = sub2(ld_pair(p0, 1), y);
+                        const f2x r2 = fma2(rx, rx, fma2(ry, ry, soft(OM, ma, mb)));
+                        const f2x inv = rsqrt2(r2);
+                        f2x f = mul2(OM, mul2(inv, mul2(inv, inv)));
+                        if (self_test) {
+                            float f0, f1;
+                            upk(f, f0, f1);
+                            f = pk(__float_as_uint(p1.z) == sa ? 0.0f : f0,
+                                   __float_as_uint(p1.w) == sb ? 0.0f : f1);
+                        }
+                        ax2 = fma2(f, rx, ax2);
+                        ay2 = fma2(f, ry, ay2);
+                    }
+                });
             }
             __syncwarp();
         };
-        int sp = 0, nn = 0, ns = 0, nf = 0;
+        int sp = 0, nn = 0, nr = 0, nf = 0;
         if (n > 1) {
             if (lane == 0) S.stack[0] = 0u;
             sp = 1;
@@ -330,104 +397,87 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             const bool has = lane < k;
             const uint32_t v = has ? S.stack[sp - k + lane] : 0u;
             sp -= k;
-            __syncwarp();
-            bool emit_node = false, emit_far = false, emit_range = false, push = false;
-            uint32_t r0 = 0, r1 = 0;
-            if (has) {
-                if (v >= nm1) {
-                    emit_range = (v - nm1) >= sys_lo && (v - nm1) < sys_hi;
-                    r0 = v - nm1;
-                    r1 = 1;
-                } else {
-                    float4 box, tr;
-                    ldg_half(&gnode[v].box, box, tr);
-                    const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
-                    bool outside = false, spans = false;
-                    if (P.num_systems > 0) {
-                        const float4 tail = __ldg(&gnode[v].tail);
-                        const uint32_t f = __float_as_uint(tail.z), e = f + __float_as_uint(tail.w);
-                        outside = e <= sys_lo || f >= sys_hi;  // another system's subtree
-                        spans = f < sys_lo || e > sys_hi;      // of several systems: always open
-                    }
-                    if (outside) {
-                        // no interaction
-                    } else if (!spans && group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2)) {
-                        r0 = v;
-                        emit_node = true;
-                        if (FAR && far_on) {
-                            // far from the group: to its local expansion
-                            const float rx = __fsub_rn(tr.x, gcx), ry = __fsub_rn(tr.y, gcy);
-                            const float R2 = __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry));
-                            emit_far = rg2 < __fmul_rn(P.far_alpha2, R2);
-                            emit_node = !emit_far;
-                        }
-                    } else if ((small & 255u) <= (uint32_t)P.leaf_size) {
-                        // (a node of several systems holds more bodies than that)
-                        emit_range = true;
-                        r0 = link_gamma(link) + 1u - (small >> 8);
-                        r1 = small & 255u;
-                    } else {
-                        push = true;
-                        r0 = link_left(link, nm1);
-                        r1 = link_right(link, nm1);
-                    }
-                }
+            // Without branches: a step is a chain of dependent instructions
+            // (~1300 cycles with them), and its lanes differ in what they find.
+            const bool inner = has & (v < nm1), leaf = has & (v >= nm1);
+            float4 box, tr;
+            ldg_half(&gnode[inner ? v : 0u].box, box, tr);
+            const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
+            bool live = inner, spans = false;
+            if (P.num_systems > 0) {
+                const float4 tail = __ldg(&gnode[inner ? v : 0u].tail);
+                const uint32_t f = __float_as_uint(tail.z), e = f + __float_as_uint(tail.w);
+                live = inner & (e > sys_lo) & (f < sys_hi);  // else another system's subtree
+                spans = (f < sys_lo) | (e > sys_hi);         // of several systems: always open
             }
-            const unsigned mp = __ballot_sync(FULL, push);
-            const int npush = 2 * __popc(mp);
-            if (sp + npush <= stack_cap) {
-                if (push) {
-                    const int p = sp + 2 * __popc(mp & lt);
-                    S.stack[p] = r1;      // right child
-                    S.stack[p + 1] = r0;  // left child on top
-                }
-                sp += npush;
-            } else if (lane == 0) {
-                atomicOr(err, kErrGroupStack);
-            }
+            const bool ok = live & !spans & group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2);
+            bool away = false;
             if (FAR) {
-                const unsigned mf = __ballot_sync(FULL, emit_far);
-                if (emit_far) S.far[nf + __popc(mf & lt)] = r0;
-                nf += __popc(mf);
+                // far from the group: to its local expansion
+                const float rx = __fsub_rn(tr.x, gcx), ry = __fsub_rn(tr.y, gcy);
+                const float R2 = __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry));
+                away = ok & (far_rg2 < __fmul_rn(P.far_alpha2, R2));
             }
-            const unsigned mn = __ballot_sync(FULL, emit_node);
-            if (emit_node) S.near[nn + __popc(mn & lt)] = r0;
+            // (a node of several systems holds more bodies than a bucket)
+            const bool bucket = live & !ok & ((small & 255u) <= (uint32_t)P.leaf_size);
+            const bool push = live & !ok & !bucket;
+            const bool range = bucket | (leaf & (v - nm1 >= sys_lo) & (v - nm1 < sys_hi));
+            const unsigned mp = __ballot_sync(FULL, push);
+            const unsigned mr = __ballot_sync(FULL, range);
+            const unsigned mn = __ballot_sync(FULL, ok & !away);
+            const unsigned mf = FAR ? __ballot_sync(FULL, away) : 0u;
+            int npush = 2 * __popc(mp);
+            if (sp + npush > stack_cap) {  // never expected
+                if (lane == 0) atomicOr(err, kErrGroupStack);
+                npush = 0;
+            } else if (push) {
+                // right child below, left child on top
+                const int p = sp + 2 * __popc(mp & lt);
+                S.stack[p] = link_right(link, nm1);
+                S.stack[p + 1] = link_left(link, nm1);
+            }
+            sp += npush;
+            if (ok) {
+                if (FAR && away) S.far[nf + __popc(mf & lt)] = v;
+                else S.near[nn + __popc(mn & lt)] = v;
+            }
+            if (range) {
+                const int p = nr + __popc(mr & lt);
+                S.first[p] = leaf ? v - nm1 : link_gamma(link) + 1u - (small >> 8);
+                S.count[p] = (unsigned char)(leaf ? 1u : small);
+            }
             nn += __popc(mn);
-            if (__any_sync(FULL, emit_range)) {
-                // Append this step's body slots: exclusive scan of the counts.
-                const uint32_t c = emit_range ? r1 : 0u;
-                uint32_t incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                const uint32_t total = __shfl_sync(FULL, incl, 31);
-                const uint32_t at = (uint32_t)ns + incl - c;
-                for (uint32_t u = 0; u < c; ++u) S.slot[at + u] = r0 + u;
-                ns += (int)total;
-            }
+            nr += __popc(mr);
+            nf += __popc(mf);
             if (counting) c_vis += (unsigned long long)k;
             __syncwarp();
             // Lists are evaluated when full, and whatever they hold once the
             // stack is empty; one call site each keeps the kernel's code
             // (and its instruction-cache footprint) small.
             const bool last = sp == 0;
+            if (!last & (nn < 32) & (nr < 32) & (!FAR | (nf < 64))) continue;
             while (nn >= 32 || (last && nn > 0)) {
                 const int cnt = nn < 32 ? nn : 32;
                 nn -= cnt;
-                if (lane < cnt) {
-                    float4 mom, tail;  // {com, mass, Sxx}, {Sxy, Syy}
-                    ldg_half(&gnode[S.near[nn + lane]].mom, mom, tail);
-                    S.ent[lane][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
+                float4 mom = make_float4(kFarAway, kFarAway, 0.f, 0.f), tail = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane < cnt) ldg_half(&gnode[S.near[nn + lane]].mom, mom, tail);
+                // {com, mass, Sxx}, {Sxy, Syy}: -Q' = tr(S) I - 3S
+                const float sxx = mom.w, sxy = tail.x, syy = tail.y, trS = sxx + syy;
+                const float nxx = trS - 3.0f * sxx, nxy = -3.0f * sxy, nyy = trS - 3.0f * syy;
+                if (full > 0) {
+                    S.nodes.ent[lane][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
+                    S.nodes.ent[lane][1] = make_float4(mom.z, mom.z, nxx, nxx);
+                    if (MP >= 2) S.nodes.ent[lane][2] = make_float4(nxy, nxy, nyy, nyy);
+                }
+                if (odd) {
+                    float* const d = reinterpret_cast<float*>(&S.nodes.ent2[lane >> 1][0]) + (lane & 1);
+                    d[0] = mom.x;
+                    d[2] = mom.y;
+                    d[4] = mom.z;
                     if (MP >= 2) {
-                        // -Q' = tr(S) I - 3S
-                        const float sxx = mom.w, sxy = tail.x, syy = tail.y, trS = sxx + syy;
-                        const float nxx = trS - 3.0f * sxx, nxy = -3.0f * sxy, nyy = trS - 3.0f * syy;
-                        S.ent[lane][1] = make_float4(mom.z, mom.z, nxx, nxx);
-                        S.ent[lane][2] = make_float4(nxy, nxy, nyy, nyy);
-                    } else {
-                        S.ent[lane][1] = make_float4(mom.z, mom.z, 0.f, 0.f);
+                        d[6] = nxx;
+                        d[8] = nxy;
+                        d[10] = nyy;
                     }
                 }
                 __syncwarp();
@@ -435,16 +485,28 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 if (counting) c_node += (unsigned long long)cnt * nvalid;
                 __syncwarp();
             }
-            if (ns >= 32 || (last && ns > 0)) {
+            while (nr >= 32 || (last && nr > 0)) {
+                // the bodies of up to 32 ranges: one exclusive scan of their counts
+                const int cnt = nr < 32 ? nr : 32;
+                nr -= cnt;
+                const uint32_t first = lane < cnt ? S.first[nr + lane] : 0u;
+                const uint32_t c = lane < cnt ? S.count[nr + lane] : 0u;
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                const int ns = (int)__shfl_sync(FULL, incl, 31);
+                for (uint32_t u = 0; u < c; ++u) S.slot[incl - c + u] = first + u;
                 if (counting) c_body += (unsigned long long)ns * nvalid;
                 eval_bodies(ns);
-                ns = 0;
             }
             if constexpr (FAR) {
-                while (nf >= 32 || (last && nf > 0)) {
-                    const int cnt = nf < 32 ? nf : 32;
+                while (nf >= 64 || (last && nf > 0)) {
+                    const int cnt = nf < 64 ? nf : 64;
                     nf -= cnt;
-                    far_batch(gnode, S.far + nf, cacc, lane, cnt, gcx, gcy, lam, eps2);
+                    far_batch(gnode, S.far + nf, cacc, lane, cnt, gcx, gcy, far_rg2, eps2);
                     if (counting) c_far += (unsigned long long)cnt;
                     far_used = true;
                 }
@@ -452,6 +514,19 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
         }
         if (counting && n > 1) c_body -= nvalid;  // each body met its own leaf once
         __syncwarp();
+        // The bodies' positions out of the pairs (nothing else keeps them).
+#pragma unroll
+        for (int k = 0; k < BPL; ++k) {
+            float lo, hi, hi2;
+            upk(X[k / 2], lo, hi);
+            bx[k] = k & 1 ? hi : lo;
+            upk(X[NP - 1], lo, hi2);
+            if (odd && k == kmax - 1) bx[k] = lo;
+            upk(Y[k / 2], lo, hi);
+            by[k] = k & 1 ? hi : lo;
+            upk(Y[NP - 1], lo, hi2);
+            if (odd && k == kmax - 1) by[k] = lo;
+        }
         // Far field: reduce the lane columns (every lane gets the sums) and
         // evaluate the local expansion at each of the lane's bodies.
         float fx[BPL], fy[BPL];
@@ -469,7 +544,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
                 c[k] = v;
             }
-            const float inv_lam = __fdiv_rn(1.0f, lam);
+            const float inv_lam = __fdiv_rn(1.0f, __fsqrt_rn(far_rg2));
 #pragma unroll
             for (int k = 0; k < BPL; ++k) {
                 if ((uint32_t)k * 32u + (uint32_t)lane >= nvalid) continue;
@@ -485,15 +560,20 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
 
         // Integrate (same modes as the exact walk).
         float ax[BPL], ay[BPL];
-        if (NP > 0) {
+        {
+            const float ox = sum_halves(AX[NP - 1]), oy = sum_halves(AY[NP - 1]);
 #pragma unroll
-            for (int q = 0; q < NP; ++q) {
-                upk(AX[q], ax[2 * q], ax[2 * q + 1]);
-                upk(AY[q], ay[2 * q], ay[2 * q + 1]);
+            for (int k = 0; k < BPL; ++k) {
+                float lo, hi;
+                upk(AX[k / 2], lo, hi);
+                ax[k] = k & 1 ? hi : lo;
+                upk(AY[k / 2], lo, hi);
+                ay[k] = k & 1 ? hi : lo;
+                if (odd && k == kmax - 1) {
+                    ax[k] = ox;
+                    ay[k] = oy;
+                }
             }
-        } else {
-            ax[0] = ax1;
-            ay[0] = ay1;
         }
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
