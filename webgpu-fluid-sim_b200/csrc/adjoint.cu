@@ -104,6 +104,7 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
                  float2* __restrict__ xbar_slot, float* __restrict__ mbar_slot,
                  const WalkParams P, uint32_t* __restrict__ err) {
     __shared__ VjpSmem smem[kVjpWarps];
+    __shared__ uint32_t s_group;
     if (step_failed(err)) return;  // the tree at these positions was not built
     const int lane = threadIdx.x & 31;
     VjpSmem& S = smem[threadIdx.x >> 5];
@@ -113,11 +114,20 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
     const uint32_t ngroups = P.group_ctr[1];
     const float th2 = __fmul_rn(P.theta, P.theta);
     const float eps2 = P.eps2, G = P.g;
+    const int turn_mask = P.split ? kVjpWarps - 1 : 0;
+    const int my_turn = P.split ? (int)(threadIdx.x >> 5) : 0;
 
     while (true) {
         uint32_t g = 0;
-        if (lane == 0) g = atomicAdd(P.group_ctr, 1u);
-        g = __shfl_sync(FULL, g, 0);
+        if (P.split) {  // the block's warps share a group, batch by batch
+            __syncthreads();
+            if (threadIdx.x == 0) s_group = atomicAdd(P.group_ctr, 1u);
+            __syncthreads();
+            g = s_group;
+        } else {
+            if (lane == 0) g = atomicAdd(P.group_ctr, 1u);
+            g = __shfl_sync(FULL, g, 0);
+        }
         if (g >= ngroups) break;
         const uint2 grp = __ldg(&groups[g]);
         const uint32_t base = grp.x, nvalid = grp.y;
@@ -313,6 +323,7 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
 
         // Same traversal as walk_group_kernel: identical interaction lists.
         int sp = 0, nn = 0, ns = 0;
+        int turn = 0;  // batches so far; a split group's are dealt to its warps
         if (n > 1) {
             if (lane == 0) S.stack[0] = 0u;
             sp = 1;
@@ -391,18 +402,18 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
             }
             __syncwarp();
             if (nn >= 32) {
-                eval_nodes(nn);
+                if ((turn++ & turn_mask) == my_turn) eval_nodes(nn);
                 nn = 0;
                 __syncwarp();
             }
             if (ns >= 32) {
-                eval_bodies(ns);
+                if ((turn++ & turn_mask) == my_turn) eval_bodies(ns);
                 ns = 0;
                 __syncwarp();
             }
         }
-        if (nn > 0) eval_nodes(nn);
-        if (ns > 0) eval_bodies(ns);
+        if (nn > 0 && (turn++ & turn_mask) == my_turn) eval_nodes(nn);
+        if (ns > 0 && (turn++ & turn_mask) == my_turn) eval_bodies(ns);
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < NP; ++q) {  // node-list part of the packed bodies
@@ -537,11 +548,14 @@ static void vjp_launch_t(const DeviceBuffers& b, const WalkParams& p, const floa
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint32_t blocks = (uint32_t)(sms * bps);
-    const uint32_t need = (b.n + kVjpWarps - 1) / kVjpWarps;
+    WalkParams q = p;
+    // (a rollout's gradient, 65k bodies, 10 groups per SM: 12.35 ms unsplit, 11.43 split)
+    q.split = split_groups(b.n, 32u * BPL, sms, 16);
+    const uint32_t need = q.split ? b.n : (b.n + kVjpWarps - 1) / kVjpWarps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     vjp_group_kernel<BPL, MP><<<blocks, kVjpWarps * 32, 0, s>>>(
-        b.gnode, b.node4, b.groups, b.ids, abar, node_adj, xbar_slot, mbar_slot, p, b.err);
+        b.gnode, b.node4, b.groups, b.ids, abar, node_adj, xbar_slot, mbar_slot, q, b.err);
 }
 
 void launch_force_vjp(const DeviceBuffers& b, const WalkParams& p, const float2* abar,

@@ -148,6 +148,7 @@ struct WalkParams {
     int multipole;    // 1 or 2
     int bpl;          // bodies per lane
     unsigned int* group_ctr;  // dynamic group counter (zeroed per step)
+    int split = 0;    // 1 = a block's warps share one group (set by the launcher)
     // ensemble: a group only sees its own system's slot range
     uint32_t num_systems;
     const uint32_t* sys_off;
@@ -264,6 +265,8 @@ void init_bound(const DeviceBuffers& b, cudaStream_t s);
 // walk.cu
 void launch_walk(const DeviceBuffers& b, const WalkParams& p, int block, cudaStream_t s);
 // walk_group.cu
+// Fewer than per_sm groups for each SM: a block's warps share one (walk and its VJP).
+bool split_groups(uint32_t n, uint32_t gmax, int sms, int per_sm);
 void launch_walk_group(const DeviceBuffers& b, const WalkParams& p, int block, cudaStream_t s);
 // shard.cu: the bodies a sharded step updated, packed / unpacked in sorted-slot order
 void launch_shard_pack(const DeviceBuffers& b, uint32_t lo, uint32_t hi, int kdk, void* chunk,

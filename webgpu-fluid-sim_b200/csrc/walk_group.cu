@@ -172,11 +172,16 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
     extern __shared__ __align__(16) unsigned char walk_smem[];
     GroupSmem* smem = reinterpret_cast<GroupSmem*>(walk_smem);
     if (step_failed(err)) return;  // the tree of this step was not built
-    const int lane = threadIdx.x & 31;
-    GroupSmem& S = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    GroupSmem& S = smem[warp];
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t n = P.n, nm1 = n - 1;
+    // Split walk (few groups): the block's warps walk one group together.  Each
+    // does the whole traversal, and evaluates every turn_mask+1-th batch.
+    const bool split = !COUNT && P.split;
+    const int turn_mask = split ? (int)(blockDim.x >> 5) - 1 : 0;
+    const int my_turn = split ? warp : 0;
     const uint32_t ngroups = P.group_ctr[1];  // written by the build kernel
     const float th2 = __fmul_rn(P.theta, P.theta);
     const float eps2 = P.eps2, ecoef = P.eps_coef;
@@ -188,13 +193,21 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
 
     while (true) {
         uint32_t g = 0;
-        if (lane == 0) g = atomicAdd(P.group_ctr, 1u);
-        g = __shfl_sync(FULL, g, 0);
+        if (split) {
+            __syncthreads();  // the previous group's sums have been read
+            if (threadIdx.x == 0) S.slot[0] = atomicAdd(P.group_ctr, 1u);
+            __syncthreads();
+            g = smem[0].slot[0];
+            __syncthreads();
+        } else {
+            if (lane == 0) g = atomicAdd(P.group_ctr, 1u);
+            g = __shfl_sync(FULL, g, 0);
+        }
         if (g >= ngroups) break;
         // A group is a subtree of <= 32 x BPL bodies: contiguous sorted slots
         // inside one Morton cell, so its box stays compact.
         const uint2 grp = __ldg(&groups[g]);
-        if (grp.x < P.slot_lo || grp.x >= P.slot_hi) continue;  // another shard's group
+        if (grp.x < P.slot_lo || grp.x >= P.slot_hi) continue;  // another shard's group (uniform)
         const uint32_t base = grp.x, nvalid = grp.y;
         const int kmax = (int)((nvalid + 31u) / 32u);  // sub-slots in use (uniform)
         // Ensemble: the slot range of this group's system (systems stay
@@ -386,6 +399,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             __syncwarp();
         };
         int sp = 0, nn = 0, nr = 0, nf = 0;
+        int turn = 0;  // batches so far
         if (n > 1) {
             if (lane == 0) S.stack[0] = 0u;
             sp = 1;
@@ -459,6 +473,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             while (nn >= 32 || (last && nn > 0)) {
                 const int cnt = nn < 32 ? nn : 32;
                 nn -= cnt;
+                if ((turn++ & turn_mask) != my_turn) continue;
                 float4 mom = make_float4(kFarAway, kFarAway, 0.f, 0.f), tail = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < cnt) ldg_half(&gnode[S.near[nn + lane]].mom, mom, tail);
                 // {com, mass, Sxx}, {Sxy, Syy}: -Q' = tr(S) I - 3S
@@ -489,6 +504,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 // the bodies of up to 32 ranges: one exclusive scan of their counts
                 const int cnt = nr < 32 ? nr : 32;
                 nr -= cnt;
+                if ((turn++ & turn_mask) != my_turn) continue;
                 const uint32_t first = lane < cnt ? S.first[nr + lane] : 0u;
                 const uint32_t c = lane < cnt ? S.count[nr + lane] : 0u;
                 uint32_t incl = c;
@@ -506,6 +522,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 while (nf >= 64 || (last && nf > 0)) {
                     const int cnt = nf < 64 ? nf : 64;
                     nf -= cnt;
+                    if ((turn++ & turn_mask) != my_turn) continue;
                     far_batch(gnode, S.far + nf, cacc, lane, cnt, gcx, gcy, far_rg2, eps2);
                     if (counting) c_far += (unsigned long long)cnt;
                     far_used = true;
@@ -577,11 +594,30 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
         }
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
+            ax[k] = far_used ? __fadd_rn(ax[k], fx[k]) : ax[k];
+            ay[k] = far_used ? __fadd_rn(ay[k], fy[k]) : ay[k];
+        }
+        if (split) {
+            // the warps' shares, added in warp order by the first one
+            float2* const mine = reinterpret_cast<float2*>(&S.nodes);
+#pragma unroll
+            for (int k = 0; k < BPL; ++k) mine[32 * k + lane] = make_float2(ax[k], ay[k]);
+            __syncthreads();
+            if (warp > 0) continue;
+            for (int w = 1; w <= turn_mask; ++w) {
+                const float2* const other = reinterpret_cast<const float2*>(&smem[w].nodes);
+#pragma unroll
+                for (int k = 0; k < BPL; ++k) {
+                    ax[k] += other[32 * k + lane].x;
+                    ay[k] += other[32 * k + lane].y;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < BPL; ++k) {
             const uint32_t s = base + (uint32_t)k * 32u + (uint32_t)lane;
             if ((uint32_t)k * 32u + (uint32_t)lane >= nvalid) continue;
-            const float axk = far_used ? __fadd_rn(ax[k], fx[k]) : ax[k];
-            const float ayk = far_used ? __fadd_rn(ay[k], fy[k]) : ay[k];
-            const float gx = P.g * axk, gy = P.g * ayk;
+            const float gx = P.g * ax[k], gy = P.g * ay[k];
             const uint32_t b = __ldg(&ids[s]);
             if (P.mode == kWalkForces) {
                 acc[b] = make_float2(gx, gy);
@@ -629,6 +665,17 @@ static cudaError_t set_walk_attributes() {
 // Largest walk block for bodies_per_lane `bpl` (its launch bound).
 int walk_group_max_block(int bpl) { return walk_max_threads(bpl >= 4 ? 4 : 2); }
 
+// With few groups the walk lasts as long as its longest one (100k bodies: 1.1k
+// groups for 2,960 resident warps), so a block's warps walk a group together:
+// below 8 groups per SM (a group holds about 0.7 of its limit).  Walk stage,
+// one warp / one block per group: 16k bodies in 64-body groups 36.7 / 28.5 us,
+// 32k 40.3 / 32.9, 65k (10 groups per SM) 52.3 / 55.3; 128-body groups without
+// the far field, 50k 157 / 77, 100k (8 per SM) 199 / 121, 200k 221 / 208; with
+// it 50k 104 / 60, 100k 114 / 98, 200k 121 / 160.
+bool split_groups(uint32_t n, uint32_t gmax, int sms, int per_sm) {
+    return (double)n < 0.7 * gmax * per_sm * sms;
+}
+
 template <int BPL, int MP, bool PL, bool FAR, bool COUNT>
 static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, cudaStream_t s) {
     static int blocks_per_sm[64][3] = {};
@@ -645,11 +692,13 @@ static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, cud
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // Persistent grid; the number of groups (<= n) is only known on the device.
     uint32_t blocks = (uint32_t)(sms * bps);
-    const uint32_t need = (b.n + warps - 1) / warps;
+    WalkParams q = p;
+    q.split = !COUNT && split_groups(b.n, 32u * BPL, sms, 8);
+    const uint32_t need = q.split ? b.n : (b.n + warps - 1) / warps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     walk_group_kernel<BPL, MP, PL, FAR, COUNT><<<blocks, warps * 32, smem, s>>>(
-        b.gnode, b.node4, b.groups, b.ids, b.pos, b.vel, b.acc, p, b.err);
+        b.gnode, b.node4, b.groups, b.ids, b.pos, b.vel, b.acc, q, b.err);
 }
 
 // The counting walk only when bh_walk_stats asks for it (p.count).
