@@ -31,18 +31,25 @@
 namespace bh {
 
 constexpr int kVjpWarps = 4;
-constexpr int kVjpStack = 384;
-constexpr int kVjpDfsAt = kVjpStack - 128;
-constexpr int kVjpSlots = 32 + 32 * kGroupMaxLeaf;
+constexpr int kVjpStack = 320;
+constexpr int kVjpDfsAt = kVjpStack - 128;  // as in the walk: >= 32 + 96 below the capacity
 
+// A warp's shared memory.  The group's bodies in pairs, read by every lane:
+// {x, x', y, y'} and the upstream adjoints {ax, ax', ay, ay'}; their position
+// adjoints, as 8 sums for every 4 bodies {x0, x1, x2, x3, y0, y1, y2, y3}.
+// Groups per SM below which a block's warps share one (a rollout's gradient,
+// limit 1 / 8 / 16 / 32: 65k bodies, 10 groups per SM, 10.9 / 10.9 / 9.67 /
+// 9.59 ms; 32k 8.63 / 7.07 / 7.08 / 7.05 ms; 16k 8.09 / 6.60 / 6.61 / 6.57).
+constexpr int kVjpSplit = 16;
+constexpr int kVjpPairs = 64;  // 128 bodies
 struct VjpSmem {
     uint32_t stack[kVjpStack];
-    // node entry j, every value duplicated so a 64-bit shared load gives an
-    // operand pair: {cx, cx, cy, cy}, {m, m, Q'xx, Q'xx}, {Q'xy, Q'xy, Q'yy, Q'yy}
-    float4 nd[kGroupList][3];
-    uint32_t nd_idx[kGroupList];  // the entry's internal node
-    uint32_t slot[kVjpSlots];
-    float4 body[32];           // staged leaf records {x, y, m, slot bits}
+    float4 body[kVjpPairs][2];
+    float xbar[kVjpPairs / 2][8];
+    uint32_t near[64];        // nodes (a step adds at most 32 to fewer than 32)
+    uint32_t first[64];       // ranges of bodies: first slot,
+    unsigned char count[64];  // and how many
+    uint32_t slot[32 * kGroupMaxLeaf];
 };
 
 // Warp sums of 8 values by recursive halving: 4 + 2 + 1 exchanges split the
@@ -73,30 +80,17 @@ __device__ __forceinline__ float warp_reduce_scatter8(float v[8]) {
     return c;
 }
 
-// Same for 4 values: lanes 8k..8k+7 hold the sum of v[k] (6 shuffles).
-__device__ __forceinline__ float warp_reduce_scatter4(float v[4]) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    const bool h4 = lane & 16, h3 = lane & 8;
-    float a[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const float keep = h4 ? v[j + 2] : v[j], send = h4 ? v[j] : v[j + 2];
-        a[j] = keep + __shfl_xor_sync(FULL, send, 16);
-    }
-    float c;
-    {
-        const float keep = h3 ? a[1] : a[0], send = h3 ? a[0] : a[1];
-        c = keep + __shfl_xor_sync(FULL, send, 8);
-    }
-    c += __shfl_xor_sync(FULL, c, 4);
-    c += __shfl_xor_sync(FULL, c, 2);
-    c += __shfl_xor_sync(FULL, c, 1);
-    return c;
-}
-
-// node_adj: 6 floats per internal node {cbar.x, cbar.y, mbar, Q'bar xx, xy, yy}
-template <int BPL, int MP>
+// node_adj: 8 floats per internal node {cbar.x, cbar.y, mbar, Q'bar xx | xy, yy, -, -}
+//
+// A lane owns one list entry (a node or a source body) of a batch of 32 and
+// runs over the group's bodies, two per packed instruction: the entry's six
+// adjoints are plain sums in its registers, one reduction of the body adjoints
+// serves 4 bodies x 32 entries, and only the bodies there are cost anything.
+// (One body per lane and one entry at a time, every entry paid a reduction of
+// its six adjoints over the warp and a partly filled group its empty lanes:
+// 65k bodies in 64-body groups 239 us a launch, 103 us now, both with the
+// block's warps sharing a group; bound by latency at that size.)
+template <int MP>
 __global__ void __launch_bounds__(kVjpWarps * 32)
 vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ node4,
                  const uint2* __restrict__ groups, const uint32_t* __restrict__ ids,
@@ -114,6 +108,9 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
     const uint32_t ngroups = P.group_ctr[1];
     const float th2 = __fmul_rn(P.theta, P.theta);
     const float eps2 = P.eps2, G = P.g;
+    const f2x E2 = pk(eps2, eps2), CM3 = pk(-3.0f, -3.0f), CM1 = pk(-1.0f, -1.0f);
+    const f2x C5 = pk(5.0f, 5.0f), C25 = pk(2.5f, 2.5f), CM175 = pk(-17.5f, -17.5f);
+    const f2x ZERO = pk(0.f, 0.f);
     const int turn_mask = P.split ? kVjpWarps - 1 : 0;
     const int my_turn = P.split ? (int)(threadIdx.x >> 5) : 0;
 
@@ -131,24 +128,27 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
         if (g >= ngroups) break;
         const uint2 grp = __ldg(&groups[g]);
         const uint32_t base = grp.x, nvalid = grp.y;
-        float bx[BPL], by[BPL], abx[BPL], aby[BPL], xbx[BPL], xby[BPL];
-        bool ok[BPL];
+        const int quads = (int)((nvalid + 3u) / 4u);
+        // ---- stage the bodies; past the end, one far away with a zero adjoint,
+        // which adds exactly zero everywhere
         float glox = INFINITY, gloy = INFINITY, ghix = -INFINITY, ghiy = -INFINITY;
-#pragma unroll
-        for (int k = 0; k < BPL; ++k) {
-            const uint32_t rel = (uint32_t)k * 32u + (uint32_t)lane;
-            ok[k] = rel < nvalid;
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 a = make_float2(0.f, 0.f);
-            if (ok[k]) {
-                r = __ldg(&node4[nm1 + base + rel]);
-                a = __ldg(&abar[__ldg(&ids[base + rel])]);
+        for (int rel = lane; rel < 4 * quads; rel += 32) {
+            float2 r = make_float2(-kFarAway, -kFarAway), a = make_float2(0.f, 0.f);
+            if ((uint32_t)rel < nvalid) {
+                const uint32_t sl = base + (uint32_t)rel;
+                const float4 o = __ldg(&node4[nm1 + sl]);
+                r = make_float2(o.x, o.y);
+                a = __ldg(&abar[__ldg(&ids[sl])]);
                 glox = fminf(glox, r.x); gloy = fminf(gloy, r.y);
                 ghix = fmaxf(ghix, r.x); ghiy = fmaxf(ghiy, r.y);
             }
-            bx[k] = r.x; by[k] = r.y;
-            abx[k] = G * a.x; aby[k] = G * a.y;  // the force carries G
-            xbx[k] = 0.f; xby[k] = 0.f;
+            float* const d = reinterpret_cast<float*>(&S.body[rel >> 1][0]) + (rel & 1);
+            d[0] = r.x;
+            d[2] = r.y;
+            d[4] = G * a.x;  // the force carries G
+            d[6] = G * a.y;
+            S.xbar[rel >> 2][rel & 3] = 0.f;
+            S.xbar[rel >> 2][4 + (rel & 3)] = 0.f;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -157,172 +157,124 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
             ghix = fmaxf(ghix, __shfl_xor_sync(FULL, ghix, o));
             ghiy = fmaxf(ghiy, __shfl_xor_sync(FULL, ghiy, o));
         }
+        __syncwarp();
 
-        // Packed pairs of the lane's bodies (BPL >= 2): positions, adjoints
-        // and the node-list part of their position adjoints.
-        constexpr int NP = BPL / 2;
-        f2x PX[NP > 0 ? NP : 1], PY[NP > 0 ? NP : 1], PAX[NP > 0 ? NP : 1], PAY[NP > 0 ? NP : 1];
-        f2x PXB[NP > 0 ? NP : 1], PYB[NP > 0 ? NP : 1];
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            PX[q] = pk(bx[2 * q], bx[2 * q + 1]);
-            PY[q] = pk(by[2 * q], by[2 * q + 1]);
-            PAX[q] = pk(abx[2 * q], abx[2 * q + 1]);
-            PAY[q] = pk(aby[2 * q], aby[2 * q + 1]);
-            PXB[q] = pk(0.f, 0.f);
-            PYB[q] = pk(0.f, 0.f);
-        }
-        const int kmax = (int)((nvalid + 31u) / 32u);  // sub-slots in use (uniform)
-
-        auto eval_nodes = [&](int cnt) {
-#pragma unroll 2
-            for (int j = 0; j < cnt; ++j) {
-                const float4 e0 = S.nd[j][0], e1 = S.nd[j][1], e2 = S.nd[j][2];
-                const uint32_t v = S.nd_idx[j];
-                float cbx = 0.f, cby = 0.f, mb = 0.f, gxx = 0.f, gxy = 0.f, gyy = 0.f;
-                if (NP > 0) {
-                    // Two bodies per instruction.  A slot past the group's end
-                    // holds a zero adjoint, so it adds exactly zero everywhere.
-                    const f2x CX = ld_pair(e0, 0), CY = ld_pair(e0, 1), M = ld_pair(e1, 0);
-                    const f2x QXX = ld_pair(e1, 1), QXY = ld_pair(e2, 0), QYY = ld_pair(e2, 1);
-                    const f2x E2 = pk(eps2, eps2), CM3 = pk(-3.0f, -3.0f), CM1 = pk(-1.0f, -1.0f);
-                    const f2x C5 = pk(5.0f, 5.0f), C25 = pk(2.5f, 2.5f), CM175 = pk(-17.5f, -17.5f);
-                    f2x CB_X = pk(0.f, 0.f), CB_Y = CB_X, MB = CB_X, GXX = CB_X, GXY = CB_X, GYY = CB_X;
-#pragma unroll
-                    for (int q = 0; q < NP; ++q) {
-                        if (2 * q >= kmax) break;
-                        const f2x rx = sub2(CX, PX[q]), ry = sub2(CY, PY[q]);
-                        const f2x sv = rsqrt2(fma2(rx, rx, fma2(ry, ry, E2)));
-                        const f2x s2 = mul2(sv, sv), s3 = mul2(sv, s2), s5 = mul2(s3, s2);
-                        const f2x ar = fma2(PAX[q], rx, mul2(PAY[q], ry));
-                        const f2x tn = mul2(mul2(s5, ar), CM3);  // -3 s^5 (ab.r)
-                        f2x rbx = mul2(M, fma2(s3, PAX[q], mul2(tn, rx)));
-                        f2x rby = mul2(M, fma2(s3, PAY[q], mul2(tn, ry)));
-                        MB = fma2(ar, s3, MB);
-                        if (MP >= 2) {
-                            const f2x s7 = mul2(s5, s2), s9 = mul2(s7, s2), s5n = mul2(s5, CM1);
-                            const f2x qrx = fma2(QXX, rx, mul2(QXY, ry));
-                            const f2x qry = fma2(QXY, rx, mul2(QYY, ry));
-                            const f2x qax = fma2(QXX, PAX[q], mul2(QXY, PAY[q]));
-                            const f2x qay = fma2(QXY, PAX[q], mul2(QYY, PAY[q]));
-                            const f2x rqr = fma2(rx, qrx, mul2(ry, qry));
-                            const f2x aqr = fma2(PAX[q], qrx, mul2(PAY[q], qry));
-                            const f2x f7 = mul2(C5, s7), h7 = mul2(C25, s7);
-                            const f2x c1 = fma2(f7, aqr, mul2(mul2(CM175, s9), mul2(rqr, ar)));
-                            const f2x f7ar = mul2(f7, ar), h7ar = mul2(h7, ar), h7rqr = mul2(h7, rqr);
-                            rbx = fma2(s5n, qax, rbx);
-                            rbx = fma2(c1, rx, rbx);
-                            rbx = fma2(f7ar, qrx, rbx);
-                            rbx = fma2(h7rqr, PAX[q], rbx);
-                            rby = fma2(s5n, qay, rby);
-                            rby = fma2(c1, ry, rby);
-                            rby = fma2(f7ar, qry, rby);
-                            rby = fma2(h7rqr, PAY[q], rby);
-                            GXX = fma2(mul2(PAX[q], rx), s5n, fma2(mul2(rx, rx), h7ar, GXX));
-                            GXY = fma2(fma2(PAX[q], ry, mul2(PAY[q], rx)), s5n,
-                                       fma2(mul2(rx, ry), f7ar, GXY));
-                            GYY = fma2(mul2(PAY[q], ry), s5n, fma2(mul2(ry, ry), h7ar, GYY));
-                        }
-                        PXB[q] = sub2(PXB[q], rbx);
-                        PYB[q] = sub2(PYB[q], rby);
-                        CB_X = add2(CB_X, rbx);
-                        CB_Y = add2(CB_Y, rby);
-                    }
-                    cbx = sum_halves(CB_X);
-                    cby = sum_halves(CB_Y);
-                    mb = sum_halves(MB);
-                    if (MP >= 2) {
-                        gxx = sum_halves(GXX);
-                        gxy = sum_halves(GXY);
-                        gyy = sum_halves(GYY);
-                    }
-                } else {
-                    const float cxn = e0.x, cyn = e0.z, mn = e1.x;
-                    const float qxx = e1.z, qxy = e2.x, qyy = e2.z;
-#pragma unroll
-                    for (int k = 0; k < BPL; ++k) {
-                        if (!ok[k]) continue;
-                        const float rx = cxn - bx[k], ry = cyn - by[k];
-                        const float s = rsqrt_ftz(fmaf(rx, rx, fmaf(ry, ry, eps2)));
-                        const float s2 = s * s, s3 = s * s2, s5 = s3 * s2;
-                        const float ar = abx[k] * rx + aby[k] * ry;
-                        float rbx = mn * (s3 * abx[k] - 3.0f * s5 * ar * rx);
-                        float rby = mn * (s3 * aby[k] - 3.0f * s5 * ar * ry);
-                        mb += ar * s3;
-                        if (MP >= 2) {
-                            const float s7 = s5 * s2, s9 = s7 * s2;
-                            const float qrx = qxx * rx + qxy * ry, qry = qxy * rx + qyy * ry;
-                            const float qax = qxx * abx[k] + qxy * aby[k], qay = qxy * abx[k] + qyy * aby[k];
-                            const float rqr = rx * qrx + ry * qry;
-                            const float aqr = abx[k] * qrx + aby[k] * qry;
-                            const float c1 = 5.0f * s7 * aqr - 17.5f * s9 * rqr * ar;
-                            rbx += -s5 * qax + c1 * rx + 5.0f * s7 * ar * qrx + 2.5f * s7 * rqr * abx[k];
-                            rby += -s5 * qay + c1 * ry + 5.0f * s7 * ar * qry + 2.5f * s7 * rqr * aby[k];
-                            gxx += -abx[k] * rx * s5 + 2.5f * rx * rx * ar * s7;
-                            gxy += -(abx[k] * ry + aby[k] * rx) * s5 + 5.0f * rx * ry * ar * s7;
-                            gyy += -aby[k] * ry * s5 + 2.5f * ry * ry * ar * s7;
-                        }
-                        xbx[k] -= rbx;
-                        xby[k] -= rby;
-                        cbx += rbx;
-                        cby += rby;
-                    }
-                }
-                if (MP >= 2) {
-                    float vals[8] = {cbx, cby, mb, gxx, gxy, gyy, 0.f, 0.f};
-                    const float tot = warp_reduce_scatter8(vals);
-                    const int q = lane >> 2;  // lanes 4q hold the sum of vals[q]
-                    if ((lane & 3) == 0 && q < 6) atomicAdd(node_adj + 6 * (size_t)v + q, tot);
-                } else {
-                    float vals[4] = {cbx, cby, mb, 0.f};
-                    const float tot = warp_reduce_scatter4(vals);
-                    const int q = lane >> 3;  // lanes 8q hold the sum of vals[q]
-                    if ((lane & 7) == 0 && q < 3) atomicAdd(node_adj + 6 * (size_t)v + q, tot);
-                }
-            }
+        // Add the warp's sums of rbar of 4 bodies (two pairs) to their adjoints.
+        auto add_quad = [&](int quad, f2x x0, f2x y0, f2x x1, f2x y1) {
+            float v[8];
+            upk(x0, v[0], v[1]);
+            upk(x1, v[2], v[3]);
+            upk(y0, v[4], v[5]);
+            upk(y1, v[6], v[7]);
+            const float tot = warp_reduce_scatter8(v);  // lanes 4k.. hold the sum of v[k]
+            if ((lane & 3) == 0) S.xbar[quad][lane >> 2] -= tot;
         };
-        auto eval_bodies = [&](int cnt) {
-            for (int j = 0; j < cnt; ++j) {
-                if ((j & 31) == 0) {  // stage the next 32 leaf records in parallel
-                    __syncwarp();
-                    if (j + lane < cnt) {
-                        const uint32_t sl = S.slot[j + lane];
-                        float4 r = __ldg(&node4[nm1 + sl]);
-                        r.w = __uint_as_float(sl);
-                        S.body[lane] = r;
-                    }
-                    __syncwarp();
+        // One node per lane (lane < cnt).
+        auto eval_nodes = [&](int cnt) {
+            const uint32_t v = lane < cnt ? S.near[lane] : 0u;
+            float4 mom = make_float4(kFarAway, kFarAway, 0.f, 0.f), tail = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane < cnt) ldg_half(&gnode[v].mom, mom, tail);  // {com, mass, Sxx}, {Sxy, Syy}
+            const float sxx = mom.w, sxy = tail.x, syy = tail.y, tr = sxx + syy;  // Q' = 3S - tr(S) I
+            const f2x CX = pk(mom.x, mom.x), CY = pk(mom.y, mom.y), M = pk(mom.z, mom.z);
+            const f2x QXX = pk(3.0f * sxx - tr, 3.0f * sxx - tr), QXY = pk(3.0f * sxy, 3.0f * sxy);
+            const f2x QYY = pk(3.0f * syy - tr, 3.0f * syy - tr);
+            f2x CB_X = ZERO, CB_Y = ZERO, MB = ZERO, GXX = ZERO, GXY = ZERO, GYY = ZERO;
+            auto pair = [&](int p, f2x& rbx, f2x& rby) {
+                const float4 b0 = S.body[p][0], b1 = S.body[p][1];
+                const f2x PAX = ld_pair(b1, 0), PAY = ld_pair(b1, 1);
+                const f2x rx = sub2(CX, ld_pair(b0, 0)), ry = sub2(CY, ld_pair(b0, 1));
+                const f2x sv = rsqrt2(fma2(rx, rx, fma2(ry, ry, E2)));
+                const f2x s2 = mul2(sv, sv), s3 = mul2(sv, s2), s5 = mul2(s3, s2);
+                const f2x ar = fma2(PAX, rx, mul2(PAY, ry));
+                const f2x tn = mul2(mul2(s5, ar), CM3);  // -3 s^5 (ab.r)
+                rbx = mul2(M, fma2(s3, PAX, mul2(tn, rx)));
+                rby = mul2(M, fma2(s3, PAY, mul2(tn, ry)));
+                MB = fma2(ar, s3, MB);
+                if (MP >= 2) {
+                    const f2x s7 = mul2(s5, s2), s9 = mul2(s7, s2), s5n = mul2(s5, CM1);
+                    const f2x qrx = fma2(QXX, rx, mul2(QXY, ry));
+                    const f2x qry = fma2(QXY, rx, mul2(QYY, ry));
+                    const f2x qax = fma2(QXX, PAX, mul2(QXY, PAY));
+                    const f2x qay = fma2(QXY, PAX, mul2(QYY, PAY));
+                    const f2x rqr = fma2(rx, qrx, mul2(ry, qry));
+                    const f2x aqr = fma2(PAX, qrx, mul2(PAY, qry));
+                    const f2x f7 = mul2(C5, s7), h7 = mul2(C25, s7);
+                    const f2x c1 = fma2(f7, aqr, mul2(mul2(CM175, s9), mul2(rqr, ar)));
+                    const f2x f7ar = mul2(f7, ar), h7ar = mul2(h7, ar), h7rqr = mul2(h7, rqr);
+                    rbx = fma2(s5n, qax, rbx);
+                    rbx = fma2(c1, rx, rbx);
+                    rbx = fma2(f7ar, qrx, rbx);
+                    rbx = fma2(h7rqr, PAX, rbx);
+                    rby = fma2(s5n, qay, rby);
+                    rby = fma2(c1, ry, rby);
+                    rby = fma2(f7ar, qry, rby);
+                    rby = fma2(h7rqr, PAY, rby);
+                    GXX = fma2(mul2(PAX, rx), s5n, fma2(mul2(rx, rx), h7ar, GXX));
+                    GXY = fma2(fma2(PAX, ry, mul2(PAY, rx)), s5n, fma2(mul2(rx, ry), f7ar, GXY));
+                    GYY = fma2(mul2(PAY, ry), s5n, fma2(mul2(ry, ry), h7ar, GYY));
                 }
-                const float4 o = S.body[j & 31];
-                const uint32_t sj = __float_as_uint(o.w);
-                float cbx = 0.f, cby = 0.f, mb = 0.f;
-#pragma unroll
-                for (int k = 0; k < BPL; ++k) {
-                    if (!ok[k] || sj == base + (uint32_t)k * 32u + (uint32_t)lane) continue;
-                    const float rx = o.x - bx[k], ry = o.y - by[k];
-                    const float s = rsqrt_ftz(fmaf(rx, rx, fmaf(ry, ry, eps2)));
-                    const float s3 = s * s * s, s5 = s3 * s * s;
-                    const float ar = abx[k] * rx + aby[k] * ry;
-                    const float rbx = o.z * (s3 * abx[k] - 3.0f * s5 * ar * rx);
-                    const float rby = o.z * (s3 * aby[k] - 3.0f * s5 * ar * ry);
-                    xbx[k] -= rbx;
-                    xby[k] -= rby;
-                    cbx += rbx;
-                    cby += rby;
-                    mb += ar * s3;
-                }
-                {
-                    float vals[4] = {cbx, cby, mb, 0.f};
-                    const float tot = warp_reduce_scatter4(vals);
-                    const int q = lane >> 3;  // lanes 8q hold the sum of vals[q]
-                    if ((lane & 7) == 0 && q < 3)
-                        atomicAdd(q == 2 ? &mbar_slot[sj] : (q == 0 ? &xbar_slot[sj].x : &xbar_slot[sj].y), tot);
-                }
+                CB_X = add2(CB_X, rbx);
+                CB_Y = add2(CB_Y, rby);
+            };
+#pragma unroll 1
+            for (int q = 0; q < quads; ++q) {
+                f2x x0, y0, x1, y1;
+                pair(2 * q, x0, y0);
+                pair(2 * q + 1, x1, y1);
+                add_quad(q, x0, y0, x1, y1);
             }
+            if (lane < cnt) {
+                float4* const na = reinterpret_cast<float4*>(node_adj + 8 * (size_t)v);
+                atomicAdd(na, make_float4(sum_halves(CB_X), sum_halves(CB_Y), sum_halves(MB),
+                                          MP >= 2 ? sum_halves(GXX) : 0.f));
+                if (MP >= 2)
+                    atomicAdd(reinterpret_cast<float2*>(na + 1),
+                              make_float2(sum_halves(GXY), sum_halves(GYY)));
+            }
+            __syncwarp();
+        };
+        // One source body per lane (lane < cnt): slots S.slot[c0 + lane].
+        auto eval_bodies = [&](int c0, int cnt) {
+            const uint32_t sj = lane < cnt ? S.slot[c0 + lane] : kSentinel;
+            float4 o = make_float4(kFarAway, kFarAway, 0.f, 0.f);
+            if (lane < cnt) o = __ldg(&node4[nm1 + sj]);
+            const f2x CX = pk(o.x, o.x), CY = pk(o.y, o.y), M = pk(o.z, o.z);
+            f2x CB_X = ZERO, CB_Y = ZERO, MB = ZERO;
+            auto pair = [&](int p, f2x& rbx, f2x& rby) {
+                const float4 b0 = S.body[p][0], b1 = S.body[p][1];
+                const f2x PAX = ld_pair(b1, 0), PAY = ld_pair(b1, 1);
+                // a body does not pull itself: seen from far away it adds nothing
+                const uint32_t at = base + 2u * (uint32_t)p;
+                float r0, r1;
+                upk(sub2(CX, ld_pair(b0, 0)), r0, r1);
+                const f2x rx = pk(sj == at ? kFarAway : r0, sj == at + 1u ? kFarAway : r1);
+                const f2x ry = sub2(CY, ld_pair(b0, 1));
+                const f2x sv = rsqrt2(fma2(rx, rx, fma2(ry, ry, E2)));
+                const f2x s2 = mul2(sv, sv), s3 = mul2(sv, s2);
+                const f2x ar = fma2(PAX, rx, mul2(PAY, ry));
+                const f2x tn = mul2(mul2(mul2(s3, s2), ar), CM3);
+                rbx = mul2(M, fma2(s3, PAX, mul2(tn, rx)));
+                rby = mul2(M, fma2(s3, PAY, mul2(tn, ry)));
+                MB = fma2(ar, s3, MB);
+                CB_X = add2(CB_X, rbx);
+                CB_Y = add2(CB_Y, rby);
+            };
+#pragma unroll 1
+            for (int q = 0; q < quads; ++q) {
+                f2x x0, y0, x1, y1;
+                pair(2 * q, x0, y0);
+                pair(2 * q + 1, x1, y1);
+                add_quad(q, x0, y0, x1, y1);
+            }
+            if (lane < cnt) {
+                atomicAdd(&xbar_slot[sj], make_float2(sum_halves(CB_X), sum_halves(CB_Y)));
+                atomicAdd(&mbar_slot[sj], sum_halves(MB));
+            }
+            __syncwarp();
         };
 
         // Same traversal as walk_group_kernel: identical interaction lists.
-        int sp = 0, nn = 0, ns = 0;
+        int sp = 0, nn = 0, nr = 0;
         int turn = 0;  // batches so far; a split group's are dealt to its warps
         if (n > 1) {
             if (lane == 0) S.stack[0] = 0u;
@@ -335,103 +287,76 @@ vjp_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ nod
             const bool has = lane < k;
             const uint32_t v = has ? S.stack[sp - k + lane] : 0u;
             sp -= k;
-            __syncwarp();
-            bool emit_node = false, emit_range = false, push = false;
-            uint32_t r0 = 0, r1 = 0;
-            if (has) {
-                if (v >= nm1) {
-                    emit_range = true;
-                    r0 = v - nm1;
-                    r1 = 1;
-                } else {
-                    float4 box, tr;
-                    ldg_half(&gnode[v].box, box, tr);
-                    const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
-                    if (group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2)) {
-                        emit_node = true;
-                    } else if ((small & 255u) <= (uint32_t)P.leaf_size) {
-                        emit_range = true;
-                        r0 = link_gamma(link) + 1u - (small >> 8);
-                        r1 = small & 255u;
-                    } else {
-                        push = true;
-                        r0 = link_left(link, nm1);
-                        r1 = link_right(link, nm1);
-                    }
-                }
+            const bool inner = has & (v < nm1), leaf = has & (v >= nm1);
+            float4 box, tr;
+            ldg_half(&gnode[inner ? v : 0u].box, box, tr);
+            const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
+            const bool ok = inner & group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2);
+            const bool bucket = inner & !ok & ((small & 255u) <= (uint32_t)P.leaf_size);
+            const bool push = inner & !ok & !bucket;
+            const bool range = bucket | leaf;
+            const unsigned mp = __ballot_sync(FULL, push);
+            const unsigned mr = __ballot_sync(FULL, range);
+            const unsigned mn = __ballot_sync(FULL, ok);
+            int npush = 2 * __popc(mp);
+            if (sp + npush > kVjpStack) {  // never expected
+                if (lane == 0) atomicOr(err, kErrGroupStack);
+                npush = 0;
+            } else if (push) {
+                const int p = sp + 2 * __popc(mp & lt);
+                S.stack[p] = link_right(link, nm1);
+                S.stack[p + 1] = link_left(link, nm1);
             }
-            const unsigned mn = __ballot_sync(FULL, emit_node);
-            if (emit_node) {
-                const int p = nn + __popc(mn & lt);
-                float4 mom, tail;  // {com, mass, Sxx}, {Sxy, Syy}
-                ldg_half(&gnode[v].mom, mom, tail);
-                const float sxx = MP >= 2 ? mom.w : 0.f, sxy = MP >= 2 ? tail.x : 0.f;
-                const float syy = MP >= 2 ? tail.y : 0.f;
-                const float tr = sxx + syy;  // Q' = 3S - tr(S) I
-                const float qxx = 3.0f * sxx - tr, qxy = 3.0f * sxy, qyy = 3.0f * syy - tr;
-                S.nd[p][0] = make_float4(mom.x, mom.x, mom.y, mom.y);
-                S.nd[p][1] = make_float4(mom.z, mom.z, qxx, qxx);
-                S.nd[p][2] = make_float4(qxy, qxy, qyy, qyy);
-                S.nd_idx[p] = v;
+            sp += npush;
+            if (ok) S.near[nn + __popc(mn & lt)] = v;
+            if (range) {
+                const int p = nr + __popc(mr & lt);
+                S.first[p] = leaf ? v - nm1 : link_gamma(link) + 1u - (small >> 8);
+                S.count[p] = (unsigned char)(leaf ? 1u : small);
             }
             nn += __popc(mn);
-            {
-                const uint32_t c = emit_range ? r1 : 0u;
+            nr += __popc(mr);
+            __syncwarp();
+            const bool last = sp == 0;
+            if (!last & (nn < 32) & (nr < 32)) continue;
+            if (nn >= 32 || (last && nn > 0)) {
+                // the first 32; the rest (fewer than 32) moves to the front
+                while (nn >= 32 || (last && nn > 0)) {
+                    const int cnt = nn < 32 ? nn : 32;
+                    if ((turn++ & turn_mask) == my_turn) eval_nodes(cnt);
+                    const uint32_t rest = cnt + lane < nn ? S.near[cnt + lane] : 0u;
+                    __syncwarp();
+                    nn -= cnt;
+                    if (lane < nn) S.near[lane] = rest;
+                    __syncwarp();
+                }
+            }
+            while (nr >= 32 || (last && nr > 0)) {
+                // the bodies of up to 32 ranges: one exclusive scan of their counts
+                const int cnt = nr < 32 ? nr : 32;
+                nr -= cnt;
+                const uint32_t f = lane < cnt ? S.first[nr + lane] : 0u;
+                const uint32_t c = lane < cnt ? S.count[nr + lane] : 0u;
                 uint32_t incl = c;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(FULL, incl, o);
                     if (lane >= o) incl += t;
                 }
-                const uint32_t total = __shfl_sync(FULL, incl, 31);
-                const uint32_t at = (uint32_t)ns + incl - c;
-                for (uint32_t u = 0; u < c; ++u) S.slot[at + u] = r0 + u;
-                ns += (int)total;
-            }
-            const unsigned mp = __ballot_sync(FULL, push);
-            const int npush = 2 * __popc(mp);
-            if (sp + npush <= kVjpStack) {
-                if (push) {
-                    const int p = sp + 2 * __popc(mp & lt);
-                    S.stack[p] = r1;
-                    S.stack[p + 1] = r0;
-                }
-                sp += npush;
-            } else if (lane == 0) {
-                atomicOr(err, kErrGroupStack);
-            }
-            __syncwarp();
-            if (nn >= 32) {
-                if ((turn++ & turn_mask) == my_turn) eval_nodes(nn);
-                nn = 0;
+                const int ns = (int)__shfl_sync(FULL, incl, 31);
+                for (uint32_t u = 0; u < c; ++u) S.slot[incl - c + u] = f + u;
                 __syncwarp();
-            }
-            if (ns >= 32) {
-                if ((turn++ & turn_mask) == my_turn) eval_bodies(ns);
-                ns = 0;
+                for (int c0 = 0; c0 < ns; c0 += 32)
+                    if ((turn++ & turn_mask) == my_turn) eval_bodies(c0, ns - c0 < 32 ? ns - c0 : 32);
                 __syncwarp();
             }
         }
-        if (nn > 0 && (turn++ & turn_mask) == my_turn) eval_nodes(nn);
-        if (ns > 0 && (turn++ & turn_mask) == my_turn) eval_bodies(ns);
         __syncwarp();
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {  // node-list part of the packed bodies
-            float lo, hi;
-            upk(PXB[q], lo, hi);
-            xbx[2 * q] += lo;
-            xbx[2 * q + 1] += hi;
-            upk(PYB[q], lo, hi);
-            xby[2 * q] += lo;
-            xby[2 * q + 1] += hi;
+        for (uint32_t rel = (uint32_t)lane; rel < nvalid; rel += 32u) {
+            const float* const xb = S.xbar[rel >> 2];
+            atomicAdd(&xbar_slot[base + rel], make_float2(xb[rel & 3u], xb[4u + (rel & 3u)]));
         }
-#pragma unroll
-        for (int k = 0; k < BPL; ++k) {
-            if (!ok[k]) continue;
-            const uint32_t s = base + (uint32_t)k * 32u + (uint32_t)lane;
-            atomicAdd(&xbar_slot[s].x, xbx[k]);
-            atomicAdd(&xbar_slot[s].y, xby[k]);
-        }
+        __syncwarp();
     }
 }
 
@@ -452,7 +377,9 @@ vjp_push_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ node
     uint32_t guard = 0;
     while (v != kSentinel && v < nm1 && guard++ < 4096u) {
         const float4 mom = __ldg(&gnode[v].mom);
-        const float* na = node_adj + 6 * (size_t)v;
+        const float4 na4 = __ldg(reinterpret_cast<const float4*>(node_adj + 8 * (size_t)v));
+        const float4 nb4 = __ldg(reinterpret_cast<const float4*>(node_adj + 8 * (size_t)v) + 1);
+        const float na[6] = {na4.x, na4.y, na4.z, na4.w, nb4.x, nb4.y};
         const double cx = mom.x, cy = mom.y, M = mom.z;
         sm += na[2];
         if (M > 0.0) {
@@ -533,7 +460,7 @@ __global__ void adj_post_kernel(const float2* __restrict__ xbar, float2* __restr
 }
 
 // ---- launchers -----------------------------------------------------------------
-template <int BPL, int MP>
+template <int MP>
 static void vjp_launch_t(const DeviceBuffers& b, const WalkParams& p, const float2* abar,
                          float* node_adj, float2* xbar_slot, float* mbar_slot, cudaStream_t s) {
     static int bps_cache[64] = {};
@@ -541,20 +468,18 @@ static void vjp_launch_t(const DeviceBuffers& b, const WalkParams& p, const floa
     cudaGetDevice(&dev);
     int& bps = bps_cache[dev & 63];
     if (bps == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, vjp_group_kernel<BPL, MP>,
-                                                      kVjpWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, vjp_group_kernel<MP>, kVjpWarps * 32, 0);
         if (bps < 1) bps = 1;
     }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint32_t blocks = (uint32_t)(sms * bps);
     WalkParams q = p;
-    // (a rollout's gradient, 65k bodies, 10 groups per SM: 12.35 ms unsplit, 11.43 split)
-    q.split = split_groups(b.n, 32u * BPL, sms, 16);
+    q.split = split_groups(b.n, 32u * (uint32_t)p.bpl, sms, kVjpSplit);
     const uint32_t need = q.split ? b.n : (b.n + kVjpWarps - 1) / kVjpWarps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
-    vjp_group_kernel<BPL, MP><<<blocks, kVjpWarps * 32, 0, s>>>(
+    vjp_group_kernel<MP><<<blocks, kVjpWarps * 32, 0, s>>>(
         b.gnode, b.node4, b.groups, b.ids, abar, node_adj, xbar_slot, mbar_slot, q, b.err);
 }
 
@@ -562,24 +487,11 @@ void launch_force_vjp(const DeviceBuffers& b, const WalkParams& p, const float2*
                       float* node_adj, float2* xbar_slot, float* mbar_slot, float2* xbar,
                       float* mbar, cudaStream_t s) {
     if (b.n == 0) return;
-    if (b.n > 1) cudaMemsetAsync(node_adj, 0, sizeof(float) * 6 * (size_t)(b.n - 1), s);
+    if (b.n > 1) cudaMemsetAsync(node_adj, 0, sizeof(float) * 8 * (size_t)(b.n - 1), s);
     cudaMemsetAsync(xbar_slot, 0, sizeof(float2) * (size_t)b.n, s);
     cudaMemsetAsync(mbar_slot, 0, sizeof(float) * (size_t)b.n, s);
-    const bool quad = p.multipole >= 2;
-    switch (p.bpl) {
-        case 1:
-            if (quad) vjp_launch_t<1, 2>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            else vjp_launch_t<1, 1>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            break;
-        case 4:
-            if (quad) vjp_launch_t<4, 2>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            else vjp_launch_t<4, 1>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            break;
-        default:
-            if (quad) vjp_launch_t<2, 2>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            else vjp_launch_t<2, 1>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
-            break;
-    }
+    if (p.multipole >= 2) vjp_launch_t<2>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
+    else vjp_launch_t<1>(b, p, abar, node_adj, xbar_slot, mbar_slot, s);
     const int blocks = (int)((b.n + 255) / 256);
     vjp_push_kernel<<<blocks, 256, 0, s>>>(b.gnode, b.node4, b.parent, b.ids, node_adj, xbar_slot,
                                           mbar_slot, xbar, mbar, b.n, p.multipole);

@@ -119,7 +119,8 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-constexpr int kGroupList = 64;  // node list of the group walk and its VJP (per warp)
+// Where an empty staged list entry lies: massless, and far from any body.
+constexpr float kFarAway = 1.0e18f;
 constexpr int kGroupMaxLeaf = 8;                // leaf_size cap of the group walk
 constexpr uint32_t kErrGroupStack = 1u << 3;    // group-walk stack overflow (never expected)
 constexpr uint32_t kErrShardCapacity = 1u << 4; // a shard's updated range exceeded its chunk

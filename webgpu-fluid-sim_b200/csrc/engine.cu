@@ -1124,7 +1124,7 @@ static int ensure_adjoint(bh_sim* s, uint32_t nck, uint32_t seg) {
     free_adjoint(s);
     const size_t nb = n ? n : 1, ni = n > 1 ? n - 1 : 1;
     Carver c;
-    size_t o_na = c.take<float>(6 * ni), o_xs = c.take<float2>(nb), o_ms = c.take<float>(nb);
+    size_t o_na = c.take<float>(8 * ni), o_xs = c.take<float2>(nb), o_ms = c.take<float>(nb);
     size_t o_ab = c.take<float2>(nb), o_xb = c.take<float2>(nb), o_vb = c.take<float2>(nb);
     size_t o_mb = c.take<float>(nb), o_ap = c.take<float2>(nb), o_tg = c.take<float2>(nb);
     size_t o_cp = c.take<float2>(nb * nck), o_cv = c.take<float2>(nb * nck);

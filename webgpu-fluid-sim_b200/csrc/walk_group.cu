@@ -80,8 +80,6 @@ namespace bh {
 // more warps reach the one-node-per-step depth guard.
 constexpr int kWalkStack = 320;
 constexpr int kWalkDfsAt = kWalkStack - 128;  // >= 32 + 96 below the capacity
-// Where an empty staged entry lies: massless, and far from any body.
-constexpr float kFarAway = 1.0e18f;
 
 // A warp's shared memory.  The lists hold node ids and body ranges: a step adds
 // at most 32 to fewer than 32 kept ones (far: 64).  32 ranges at a time are
