@@ -362,7 +362,7 @@ int bh_build_hierarchy_static(const void* sorted_codes, int32_t morton_bits,
  * potential energy W = -G sum_{i<j} m_i m_j / sqrt(r_ij^2 + eps_ij^2) with
  * the softening of the handle's force law (Plummer eps, or the reference's
  * eps_ij^2 = epsMult^2 G dt max(m_i, m_j), barnes_hut.wgsl:90-92).  W is an
- * O(N^2) direct sum (pair terms in FP32, sums in FP64; ~0.1 s at 800k bodies
+ * O(N^2) direct sum (pair terms in FP32, sums in FP64; 75 ms at 800k bodies
  * on a B200); potential_energy is NaN and pairs 0 when it is skipped.
  * Synchronises the handle's stream. */
 typedef struct bh_diagnostics {

@@ -225,6 +225,7 @@ struct BodyView {
     const float2* pos = nullptr;
     const float2* vel = nullptr;
     const float* radius = nullptr;
+    double* diag = nullptr;  // 8 sums of the diagnostics
     uint32_t n = 0;
     cudaStream_t stream = nullptr;
     int device = 0;

@@ -11,12 +11,11 @@
 // so that W is the potential whose gradient is the walk's direct-sum force.
 //
 // moments_kernel: grid-stride FP64 sums, warp shuffles, one FP64 atomic per
-// block and quantity.  potential_kernel: the O(N^2) pair sum, tiled through
-// shared memory (256 bodies per tile): each thread owns one body, sums a
-// tile's terms m_j / r_ij in FP32 (rsqrt, relative error ~1e-7 per term) and
-// adds each tile's sum into an FP64 accumulator; blocks add m_i-weighted sums
-// with one FP64 atomic.  About 10 operations per pair: 800k bodies take
-// ~0.1 s, so W is for diagnostics, not for every step.
+// block and quantity.  potential_kernel: the O(N^2) pair sum over unordered
+// pairs, tiled through shared memory: a tile's terms m_j / r_ij of a body are
+// summed in FP32 (256 at most; rsqrt, relative error ~1e-7 per term) and each
+// tile's sum is added into an FP64 accumulator; blocks add m_i-weighted sums
+// with one FP64 atomic.  W is for diagnostics, not for every step.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -24,6 +23,7 @@
 
 #include "bh.h"
 #include "bh_internal.cuh"
+#include "packed.cuh"
 
 namespace bh {
 
@@ -67,48 +67,112 @@ moments_kernel(const float* __restrict__ mass, const float2* __restrict__ pos,
     }
 }
 
+// Each unordered pair once: a block owns kPotBlock bodies i (kPotPerThread per
+// thread, two per packed instruction) and a run of tiles of kPotTile bodies j;
+// tiles below its own bodies are another block's, tiles that overlap them take
+// the pairs with j > i.  Bound by the reciprocal square roots: 16 a clock and
+// SM, one per pair; everything else of a pair takes fewer slots than that.
+// A call (B200; every ordered pair with scalar arithmetic, now; the square
+// roots alone): 200k bodies 24.0 / 5.0 / 4.3 ms, 800k 429 / 75 / 69 ms.
+constexpr int kPotPerThread = 4;
+constexpr uint32_t kPotBlock = kDiagThreads * kPotPerThread;
+constexpr uint32_t kPotTile = kDiagThreads;
+
+template <bool PLUMMER>
 __global__ void __launch_bounds__(kDiagThreads)
 potential_kernel(const float* __restrict__ mass, const float2* __restrict__ pos, uint32_t n,
-                 int plummer, float eps2, float eps_coef, double* __restrict__ out) {
-    __shared__ float4 tile[kDiagThreads];  // {x, y, m, 0}
+                 float eps2, float eps_coef, uint32_t tiles_per_block, double* __restrict__ out) {
+    __shared__ float4 tile[kPotTile][2];  // {x, x, y, y}, {m, m, 0, 0}
     __shared__ double s[kDiagThreads / 32];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float xi = 0.0f, yi = 0.0f, mi = 0.0f;
-    if (i < n) {
-        const float2 p = pos[i];
-        xi = p.x;
-        yi = p.y;
-        mi = mass[i];
+    constexpr int NP = kPotPerThread / 2;
+    const uint32_t i0 = blockIdx.x * kPotBlock;
+    const uint32_t own = i0 / kPotTile;  // first tile with a pair j > i
+    const uint32_t tiles = (n + kPotTile - 1) / kPotTile;
+    const uint64_t at = (uint64_t)own + (uint64_t)blockIdx.y * tiles_per_block;
+    if (at >= tiles) return;  // the shorter runs of later blocks
+    const uint32_t t0 = (uint32_t)at;
+    const uint32_t t1 = t0 + tiles_per_block < tiles ? t0 + tiles_per_block : tiles;
+    f2x X[NP], Y[NP], A[NP];
+    float mi[kPotPerThread];
+    double acc[kPotPerThread];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        float px[2], py[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = i0 + (uint32_t)(2 * q + h) * kDiagThreads + threadIdx.x;
+            const bool ok = i < n;
+            const float2 p = ok ? pos[i] : make_float2(-kFarAway, -kFarAway);
+            px[h] = p.x;
+            py[h] = p.y;
+            mi[2 * q + h] = ok ? mass[i] : 0.0f;
+            acc[2 * q + h] = 0.0;
+        }
+        X[q] = pk(px[0], px[1]);
+        Y[q] = pk(py[0], py[1]);
     }
-    double acc = 0.0;
-    for (uint32_t t0 = 0; t0 < n; t0 += kDiagThreads) {
+    const f2x E2 = pk(eps2, eps2);
+    for (uint32_t t = t0; t < t1; ++t) {
         __syncthreads();
-        const uint32_t j = t0 + threadIdx.x;
-        if (j < n) {
-            const float2 p = pos[j];
-            tile[threadIdx.x] = make_float4(p.x, p.y, mass[j], 0.0f);
-        } else {
-            tile[threadIdx.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        {
+            const uint32_t j = t * kPotTile + threadIdx.x;
+            const float2 p = j < n ? pos[j] : make_float2(kFarAway, kFarAway);
+            const float m = j < n ? mass[j] : 0.0f;
+            tile[threadIdx.x][0] = make_float4(p.x, p.x, p.y, p.y);
+            tile[threadIdx.x][1] = make_float4(m, m, 0.0f, 0.0f);
         }
         __syncthreads();
-        if (i < n) {
-            const uint32_t cnt = (n - t0) < (uint32_t)kDiagThreads ? (n - t0) : (uint32_t)kDiagThreads;
-            float sum = 0.0f;
-            for (uint32_t k = 0; k < cnt; ++k) {
-                const float4 o = tile[k];
-                const float dx = o.x - xi, dy = o.y - yi;
-                const float e2 = plummer ? eps2 : eps_coef * fmaxf(mi, o.z);
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, e2));
-                const float term = (t0 + k == i || !(r2 > 0.0f)) ? 0.0f : o.z * rsqrt_ftz(r2);
-                sum += term;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) A[q] = pk(0.0f, 0.0f);
+        const bool overlap = t * kPotTile < i0 + kPotBlock;
+        auto pairs = [&](int k, bool after0, bool after1, int q) {
+            const float4 o = tile[k][0];
+            const f2x M = ld_pair(tile[k][1], 0);
+            const f2x dx = sub2(ld_pair(o, 0), X[q]), dy = sub2(ld_pair(o, 1), Y[q]);
+            f2x e2 = E2;
+            if (!PLUMMER) {
+                float m, m1;
+                upk(M, m, m1);
+                e2 = pk(eps_coef * fmaxf(mi[2 * q], m), eps_coef * fmaxf(mi[2 * q + 1], m));
             }
-            acc += (double)sum;
+            const f2x r2 = fma2(dx, dx, fma2(dy, dy, e2));
+            float a, b;
+            upk(r2, a, b);
+            // coincident unsoftened pairs (and ones without a distance) count nothing
+            const f2x inv = pk(a > 0.0f && after0 ? rsqrt_ftz(a) : 0.0f,
+                               b > 0.0f && after1 ? rsqrt_ftz(b) : 0.0f);
+            A[q] = fma2(M, inv, A[q]);
+        };
+        if (!overlap) {
+#pragma unroll 16
+            for (int k = 0; k < (int)kPotTile; ++k)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) pairs(k, true, true, q);
+        } else {
+#pragma unroll 2
+            for (int k = 0; k < (int)kPotTile; ++k) {
+                const uint32_t j = t * kPotTile + (uint32_t)k;
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    const uint32_t i = i0 + (uint32_t)(2 * q) * kDiagThreads + threadIdx.x;
+                    pairs(k, j > i, j > i + kDiagThreads, q);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            float a, b;
+            upk(A[q], a, b);
+            acc[2 * q] += (double)a;
+            acc[2 * q + 1] += (double)b;
         }
     }
-    acc *= (double)mi;
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < kPotPerThread; ++k) sum += acc[k] * (double)mi[k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double t = warp_sum_d(acc);
-    if (lane == 0) s[warp] = t;
+    const double tot = warp_sum_d(sum);
+    if (lane == 0) s[warp] = tot;
     __syncthreads();
     if (threadIdx.x == 0) {
         double b = 0.0;
@@ -184,9 +248,9 @@ extern "C" int bh_diagnostics_compute(bh_sim* sim, int with_potential, bh_diagno
     if (e != cudaSuccess) return dfail(BH_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
     double h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (v.n > 0) {
-        double* d = nullptr;
-        e = cudaMallocAsync((void**)&d, sizeof(h), v.stream);
-        if (e != cudaSuccess) return dfail(BH_ERR_CUDA, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+        // The handle's own 64 bytes: an allocation per call cost more than the
+        // sums of 10k bodies (call 549 -> 65 us).
+        double* const d = v.diag;
         cudaMemsetAsync(d, 0, sizeof(h), v.stream);
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, v.device);
@@ -200,12 +264,24 @@ extern "C" int bh_diagnostics_compute(bh_sim* sim, int with_potential, bh_diagno
             // (epsMult sqrt(G dt m))^2, barnes_hut.wgsl:90-92
             const float coef = cfg.epsilon_multiplier * cfg.epsilon_multiplier * cfg.grav_constant *
                                cfg.delta_time;
-            bh::potential_kernel<<<need, bh::kDiagThreads, 0, v.stream>>>(v.mass, v.pos, v.n, plummer,
-                                                                           eps2, coef, d + 7);
+            const uint32_t own = (v.n + bh::kPotBlock - 1) / bh::kPotBlock;
+            const uint32_t tiles = (v.n + bh::kPotTile - 1) / bh::kPotTile;
+            // runs of up to 64 tiles, shorter where that leaves fewer than
+            // about 16 blocks per SM (half of the grid lies below the diagonal)
+            uint64_t run = (uint64_t)own * tiles / (32u * (uint64_t)sms);
+            if (run < 1) run = 1;
+            if (run > 64) run = 64;
+            if (run < tiles / 65535u + 1u) run = tiles / 65535u + 1u;  // grid.y's limit
+            const dim3 grid(own, (uint32_t)((tiles + run - 1) / run));
+            if (plummer)
+                bh::potential_kernel<true><<<grid, bh::kDiagThreads, 0, v.stream>>>(
+                    v.mass, v.pos, v.n, eps2, coef, (uint32_t)run, d + 7);
+            else
+                bh::potential_kernel<false><<<grid, bh::kDiagThreads, 0, v.stream>>>(
+                    v.mass, v.pos, v.n, eps2, coef, (uint32_t)run, d + 7);
         }
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, v.stream);
-        cudaFreeAsync(d, v.stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
         if (e != cudaSuccess) return dfail(BH_ERR_CUDA, std::string("diagnostics: ") + cudaGetErrorString(e));
     }
@@ -216,8 +292,7 @@ extern "C" int bh_diagnostics_compute(bh_sim* sim, int with_potential, bh_diagno
     out->momentum[1] = h[4];
     out->angular_momentum = h[5];
     out->kinetic_energy = 0.5 * h[6];
-    // each pair was summed from both sides
-    out->potential_energy = with_potential ? -0.5 * (double)cfg.grav_constant * h[7] : NAN;
+    out->potential_energy = with_potential ? -(double)cfg.grav_constant * h[7] : NAN;
     out->pairs = (with_potential && v.n > 1) ? (uint64_t)v.n * (v.n - 1) / 2 : 0;
     return BH_OK;
 }

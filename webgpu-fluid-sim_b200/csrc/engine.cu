@@ -97,6 +97,7 @@ struct bh_sim {
     // ensemble of independent systems (empty: one system)
     std::vector<uint32_t> sys_sizes;
     std::string err;
+    double* diag = nullptr;        // sums of bh_diagnostics_compute (in the arena)
     uint32_t* err_host = nullptr;  // page-locked copy of the device error word
 };
 
@@ -147,6 +148,7 @@ bool sim_body_view(const bh_sim* s, BodyView* out) {
     out->pos = s->b.pos;
     out->vel = s->b.vel;
     out->radius = s->b.radius;
+    out->diag = s->diag;
     out->n = s->b.n;
     out->stream = s->stream;
     out->device = s->device;
@@ -349,6 +351,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     size_t o_scr = c.take<bh::StepScratch>(1);
     size_t o_status = c.take<uint32_t>((size_t)kb * (tiles ? tiles : 1) * bh::kRadix);
     size_t o_err = c.take<uint32_t>(1);
+    size_t o_diag = c.take<double>(8);
     size_t o_soff = E ? c.take<uint32_t>(E + 1) : 0, o_bsys = E ? c.take<uint32_t>(nb) : 0;
     size_t o_sbox = E ? c.take<uint32_t>(4 * (size_t)E) : 0;
     // staged uploads and the asynchronous download's snapshot
@@ -393,6 +396,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     b.status = (uint32_t*)(a + o_status);
     b.tiles = tiles;
     b.err = (uint32_t*)(a + o_err);
+    s->diag = (double*)(a + o_diag);
     b.spin_cap = s->debug_spin_cap ? s->debug_spin_cap : bh::kSpinCapDefault;
     b.debug_flags = s->debug_flags;
     s->up[bh_sim::kPos].buf = a + o_stpos;
