@@ -20,16 +20,8 @@ constexpr int kStackSize = 256;  // barnes_hut.wgsl:67
 #endif
 constexpr uint32_t kFp64MinBodies = BH_FP64_MIN_BODIES;
 
-// Sort tiling (a tile is kSortThreads x kSortItems keys).
-#ifndef BH_SORT_THREADS
-#define BH_SORT_THREADS 512
-#endif
-#ifndef BH_SORT_ITEMS
-#define BH_SORT_ITEMS 12
-#endif
-constexpr int kSortThreads = BH_SORT_THREADS;
-constexpr int kSortItems = BH_SORT_ITEMS;
-constexpr int kSortTile = kSortThreads * kSortItems;
+// Sort tiling: a tile is kSortThreads x items keys (sort_items).
+constexpr int kSortThreads = 512;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 256;
 
@@ -252,6 +244,7 @@ int walk_group_max_block(int bpl);
 // tree.cu: the hierarchy build's dynamic shared memory limit (per device)
 cudaError_t build_init_attributes();
 int sort_passes(const DeviceBuffers& b);
+uint32_t sort_tiles(uint32_t n);  // tiles of the sort of n keys
 // tree.cu
 void launch_build_fill(const DeviceBuffers& b, int fp64_levels, cudaStream_t s);
 // Bodies from which the build runs as two kernels (local phase + frontier climb).

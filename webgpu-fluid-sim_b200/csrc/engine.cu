@@ -335,7 +335,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     // Ensembles key (system << 32) | 32-bit Morton code: 64-bit keys.
     const int kb = E ? 8 : s->cfg.morton_bits / 8;
     const size_t nn = n ? 2 * (size_t)n - 1 : 1, ni = n > 1 ? (size_t)n - 1 : 1, nb = n ? n : 1;
-    const uint32_t tiles = (uint32_t)((n + bh::kSortTile - 1) / bh::kSortTile);
+    const uint32_t tiles = bh::sort_tiles(n);
     Carver c;
     size_t o_mass = c.take<float>(nb), o_pos = c.take<float2>(nb), o_vel = c.take<float2>(nb);
     size_t o_acc = c.take<float2>(nb), o_rad = c.take<float>(nb), o_xm = c.take<float4>(nb);

@@ -9,7 +9,7 @@
 // Design (onesweep, one kernel per 8-bit digit):
 //  - The digit histograms of every pass come from the encode kernel, so each
 //    pass reads its keys exactly once.
-//  - A CTA takes the next tile (kSortTile keys) from an atomic counter (so lower
+//  - A CTA takes the next tile (512 threads x sort_items keys) from an atomic counter (so lower
 //    tiles are always already running), ranks its keys warp by warp with a
 //    ballot multisplit (stable: item-major, lane-minor = memory order),
 //    publishes its per-digit counts, stages the tile in shared memory in
@@ -62,13 +62,14 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_tot)
 #define BH_SORT_MIN_BLOCKS 2
 #endif
 
-template <typename K, bool FIRST>
+template <typename K, int kSortItems, bool FIRST>
 __global__ void __launch_bounds__(kSortThreads, BH_SORT_MIN_BLOCKS)
 onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_in,
                 K* __restrict__ keys_out, uint32_t* __restrict__ ids_out, uint32_t n, int pass,
                 StepScratch* __restrict__ scratch, uint32_t* __restrict__ status, uint32_t tiles,
                 uint32_t* __restrict__ err, uint32_t spin_cap, uint32_t debug_flags) {
     constexpr int W = kSortThreads / 32;
+    constexpr int kSortTile = kSortThreads * kSortItems;
     __shared__ uint32_t s_whist[W][kRadix];
     __shared__ uint32_t s_tile_excl[kRadix];
     __shared__ uint32_t s_gbase[kRadix];
@@ -232,9 +233,24 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
 // known to be zero (ensemble keys: system id above a 32-bit Morton code).
 int sort_passes(const DeviceBuffers& b) { return b.sort_passes > 0 ? b.sort_passes : b.key_bytes; }
 
-template <typename K>
+// Keys per thread.  Many keys keep a large sort's tiles (and its look-back) few;
+// a small one has fewer tiles than SMs, so it lasts as long as one tile: short
+// tiles below 450k keys.  All passes, 12 / 6 / 3 / 2 / 1 keys (us): 2k bodies
+// 33 / 27 / 21 / 19 / 19, 16k 43 / 35 / 25 / 25 / 25, 100k 45 / 39 / 31 / 31 /
+// 35, 400k 50 / 45 / 45 / 53 / 78, 800k 53 / 55 / 68 / 83 / 132; 64-bit keys
+// 100k 92 / 76 / 58 / 57 / 64, 300k 101 / 85 / 76 / 80 / 119, 1M 136 / 143 /
+// 154 / 193 / 317.
+constexpr int kSmallItems = 3, kLargeItems = 12;
+constexpr uint32_t kSmallSort = 450000;
+static int sort_items(uint32_t n) { return n < kSmallSort ? kSmallItems : kLargeItems; }
+uint32_t sort_tiles(uint32_t n) {
+    const uint32_t tile = (uint32_t)(kSortThreads * sort_items(n));
+    return (uint32_t)(((uint64_t)n + tile - 1) / tile);
+}
+
+template <typename K, int ITEMS>
 static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
-    const size_t smem = (size_t)kSortTile * (sizeof(K) + sizeof(uint32_t));
+    const size_t smem = (size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t));
     const int passes = sort_passes(b);
     K* kin = (K*)b.codes;
     K* kout = (K*)b.codes_alt;
@@ -242,11 +258,11 @@ static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
     uint32_t* iout = b.ids_alt;
     for (int p = 0; p < passes; ++p) {
         if (p == 0)
-            onesweep_kernel<K, true><<<b.tiles, kSortThreads, smem, s>>>(
+            onesweep_kernel<K, ITEMS, true><<<b.tiles, kSortThreads, smem, s>>>(
                 kin, nullptr, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
                 b.debug_flags);
         else
-            onesweep_kernel<K, false><<<b.tiles, kSortThreads, smem, s>>>(
+            onesweep_kernel<K, ITEMS, false><<<b.tiles, kSortThreads, smem, s>>>(
                 kin, iin, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
                 b.debug_flags);
         K* tk = kin; kin = kout; kout = tk;
@@ -254,28 +270,36 @@ static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
     }
 }
 
-template <typename K>
+template <typename K, int ITEMS>
 static cudaError_t set_sort_attributes() {
-    const int smem = (int)((size_t)kSortTile * (sizeof(K) + sizeof(uint32_t)));
-    cudaError_t e = cudaFuncSetAttribute(onesweep_kernel<K, true>,
+    const int smem = (int)((size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t)));
+    cudaError_t e = cudaFuncSetAttribute(onesweep_kernel<K, ITEMS, true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(onesweep_kernel<K, false>,
+    return cudaFuncSetAttribute(onesweep_kernel<K, ITEMS, false>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
 // Opt the sort kernels into more than 48 KB of dynamic shared memory on the
 // current device (called once per device before any launch or capture).
 cudaError_t sort_init_attributes() {
-    cudaError_t e = set_sort_attributes<uint32_t>();
-    if (e != cudaSuccess) return e;
-    return set_sort_attributes<uint64_t>();
+    cudaError_t e;
+    if ((e = set_sort_attributes<uint32_t, kLargeItems>()) != cudaSuccess) return e;
+    if ((e = set_sort_attributes<uint64_t, kLargeItems>()) != cudaSuccess) return e;
+    if ((e = set_sort_attributes<uint32_t, kSmallItems>()) != cudaSuccess) return e;
+    return set_sort_attributes<uint64_t, kSmallItems>();
 }
 
 void launch_sort(const DeviceBuffers& b, cudaStream_t s) {
     if (b.n == 0) return;
-    if (b.key_bytes == 8) sort_impl<uint64_t>(b, s);
-    else sort_impl<uint32_t>(b, s);
+    const bool small = sort_items(b.n) == kSmallItems;
+    if (b.key_bytes == 8) {
+        if (small) sort_impl<uint64_t, kSmallItems>(b, s);
+        else sort_impl<uint64_t, kLargeItems>(b, s);
+    } else {
+        if (small) sort_impl<uint32_t, kSmallItems>(b, s);
+        else sort_impl<uint32_t, kLargeItems>(b, s);
+    }
 }
 
 }  // namespace bh
