@@ -158,73 +158,12 @@ struct BuildShared {
     int suf[B];             // suf[q] = min of d[q+1..B]
     unsigned char local[B + 1];
     uint32_t bound[B + 1];  // exchange slots of the local splits
-    // Leaves by slot - B0 and local internal nodes by index - B0: float4
-    // records ({x, y, m, 0}; {cx, cy, m, 0}, box, {S, 0}) for the split
-    // build's large CTAs, separate float arrays ([3][B] {m, x, y}; [10][B]
-    // {m, cx, cy, box, S}) for the fused build's small ones -- each measured
-    // the faster layout for its kernel.
-    static constexpr bool kVec = B >= 256;
-    alignas(16) float leaf[kVec ? 4 * B : 3 * B];
-    alignas(16) float rec[kVec ? 12 * B : 10 * B];
+    float4 leaf[B];         // {x, y, m, 0} by slot - B0
+    // local internal nodes by index - B0: {cx, cy, m, link bits}, box,
+    // {Sxx, Sxy, Syy, body count bits (0: no such node)}, and first slot - B0
+    float4 mom[B], box[B], quad[B];
+    unsigned short first[B];
 };
-
-// Record access in either layout of BuildShared.  Reads follow the block
-// fence after the exchange and writes precede the next one, which orders
-// them (the fence is also a compiler barrier); the separate arrays are read
-// and written through volatile pointers as before.
-template <typename K, int B>
-__device__ __forceinline__ float4 shared_leaf(BuildShared<K, B>* S, int k) {
-    if constexpr (BuildShared<K, B>::kVec) return reinterpret_cast<const float4*>(S->leaf)[k];
-    const volatile float* v = S->leaf;
-    return make_float4(v[B + k], v[2 * B + k], v[k], 0.f);
-}
-template <typename K, int B>
-__device__ __forceinline__ void put_leaf(BuildShared<K, B>* S, int k, float4 r) {
-    if constexpr (BuildShared<K, B>::kVec) {
-        reinterpret_cast<float4*>(S->leaf)[k] = r;
-    } else {
-        S->leaf[k] = r.z;
-        S->leaf[B + k] = r.x;
-        S->leaf[2 * B + k] = r.y;
-    }
-}
-template <typename K, int B>
-__device__ __forceinline__ void shared_rec(BuildShared<K, B>* S, int k, float4& mom, float4& box,
-                                           float4& quad) {
-    if constexpr (BuildShared<K, B>::kVec) {
-        const float4* r = reinterpret_cast<const float4*>(S->rec);
-        mom = r[k];
-        box = r[B + k];
-        quad = r[2 * B + k];
-    } else {
-        const volatile float* v = S->rec;
-        mom = make_float4(v[B + k], v[2 * B + k], v[k], 0.f);
-        box = make_float4(v[3 * B + k], v[4 * B + k], v[5 * B + k], v[6 * B + k]);
-        quad = make_float4(v[7 * B + k], v[8 * B + k], v[9 * B + k], 0.f);
-    }
-}
-template <typename K, int B>
-__device__ __forceinline__ void put_rec(BuildShared<K, B>* S, int k, float4 mom, float4 box,
-                                        float4 quad) {
-    if constexpr (BuildShared<K, B>::kVec) {
-        float4* r = reinterpret_cast<float4*>(S->rec);
-        r[k] = mom;
-        r[B + k] = box;
-        r[2 * B + k] = quad;
-    } else {
-        volatile float* v = S->rec;
-        v[k] = mom.z;
-        v[B + k] = mom.x;
-        v[2 * B + k] = mom.y;
-        v[3 * B + k] = box.x;
-        v[4 * B + k] = box.y;
-        v[5 * B + k] = box.z;
-        v[6 * B + k] = box.w;
-        v[7 * B + k] = quad.x;
-        v[8 * B + k] = quad.y;
-        v[9 * B + k] = quad.z;
-    }
-}
 
 // The node a climbing thread currently owns: its slot range, the deltas at
 // the range's two boundaries, and its record.
@@ -235,222 +174,218 @@ struct Climb {
     float lox, loy, hix, hiy;
     float sxx, sxy, syy;       // second moments about the COM (group walk)
     double dm, dmx, dmy;       // valid when the node has >= kFp64MinBodies bodies
-    bool local;                // still in the block-local phase
 };
 
-// One level of the climb from the node in `c`: returns false when this thread
-// is the first to arrive at the split (it stops; the sibling's thread goes
-// on) or has created the root, else true with `c` holding the parent.
-//   LOCAL: the thread starts in the block-local phase (shared memory `S` of
-//          the CTA owning slots [B0, B0 + B)).
-//   STOP:  at the first split that is not local, record the node in the
-//          frontier list and stop (the split build's first kernel); else go
-//          on with the device-scope protocol (fused build, second kernel).
-template <typename K, int B, bool LOCAL, bool STOP>
-__device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c, BuildShared<K, B>* S,
-                                           uint32_t B0) {
-    const uint32_t n = A.n, nm1 = n - 1;
-    bool local = LOCAL && c.local;
-    {
+// Mass, centre and second moments of the parent of two nodes (f32 path):
+//   M = m_a + m_b;  com = (c_a m_a + c_b m_b) / M  (0 if M <= 0)   (lbvh.wgsl:216-224)
+//   S = sum_c S_c + m_c d_c d_c^T, d_c = c_c - com (leaves: S_c = 0).
+// Each sum joins two terms with one IEEE addition, which is commutative, so
+// the children need no ordering.
+__device__ __forceinline__ void join_centres(float ma, float ax, float ay, float mb, float bx,
+                                             float by, float& tm, float& cx, float& cy) {
+    tm = __fadd_rn(ma, mb);
+    cx = 0.0f;
+    cy = 0.0f;
+    if (tm > 0.0f) {
+        const float inv = __frcp_rn(tm);
+        cx = div_by(__fadd_rn(__fmul_rn(ax, ma), __fmul_rn(bx, mb)), tm, inv);
+        cy = div_by(__fadd_rn(__fmul_rn(ay, ma), __fmul_rn(by, mb)), tm, inv);
+    }
+}
+__device__ __forceinline__ void join_moments(float ma, float ax, float ay, float mb, float bx,
+                                             float by, float cx, float cy, const float4& sq,
+                                             float& sxx, float& sxy, float& syy) {
+    const float dax = __fsub_rn(ax, cx), day = __fsub_rn(ay, cy);
+    const float dbx = __fsub_rn(bx, cx), dby = __fsub_rn(by, cy);
+    const float madx = __fmul_rn(ma, dax), mady = __fmul_rn(ma, day);
+    const float mbdx = __fmul_rn(mb, dbx), mbdy = __fmul_rn(mb, dby);
+    sxx = __fadd_rn(__fmaf_rn(madx, dax, sxx), __fmaf_rn(mbdx, dbx, sq.x));
+    sxy = __fadd_rn(__fmaf_rn(madx, day, sxy), __fmaf_rn(mbdx, dby, sq.y));
+    syy = __fadd_rn(__fmaf_rn(mady, day, syy), __fmaf_rn(mbdy, dby, sq.z));
+}
+
+// Write node `pidx` over slots [pl, pl + cnt) to the tree arrays: its record,
+// its children's parent entries, and the walk groups it ends (a child is a
+// maximal subtree of <= gmax bodies when its parent is too big; the whole tree
+// is one when n <= gmax).
+template <typename K>
+__device__ __forceinline__ void emit_node(const BuildArgs<K>& A, uint32_t pidx, uint32_t pl,
+                                          uint32_t cnt, uint32_t link, float cx, float cy, float m,
+                                          float4 box, float sxx, float sxy, float syy) {
+    const uint32_t nm1 = A.n - 1;
+    const uint32_t gamma = link_gamma(link);
+    const uint32_t li = link_left(link, nm1), ri = link_right(link, nm1);
+    if (A.gnode) {
+        GNode* const g = &A.gnode[pidx];
+        st_half(&g->mom, make_float4(cx, cy, m, sxx),
+                make_float4(sxy, syy, __uint_as_float(pl), __uint_as_float(cnt)));
+        st_half(&g->box, box,
+                make_float4(cx, cy, __uint_as_float(link),
+                            __uint_as_float(pack_small(cnt, gamma - pl + 1u))));
+    } else {
+        // Reference layout (lbvh.wgsl:12-22, split into hot and cold arrays).
+        // With the packed records it is derived on request (ref_layout_kernel).
+        const float len = fmaxf(__fsub_rn(box.z, box.x), __fsub_rn(box.w, box.y));
+        A.node4[pidx] = make_float4(cx, cy, m, len);
+        A.aabb[pidx] = box;
+        A.children[pidx] = make_uint2(li, ri);
+        A.range[pidx] = make_uint2(pl, pl + cnt - 1u);
+    }
+    A.parent[li] = pidx;
+    A.parent[ri] = pidx;
+    if (cnt == A.n) A.parent[0] = kSentinel;  // the root (lbvh.wgsl:159-161)
+    if (A.groups) {
+        if (cnt > A.gmax) {
+            const uint32_t lcnt = gamma - pl + 1, rcnt = cnt - lcnt;
+            if (lcnt <= A.gmax) A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(pl, lcnt);
+            if (rcnt <= A.gmax) A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(gamma + 1, rcnt);
+        } else if (cnt == A.n) {
+            A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(0u, A.n);
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t make_link(uint32_t gamma, bool left_leaf, bool right_leaf) {
+    return gamma | (left_leaf ? kLinkLeftLeaf : 0u) | (right_leaf ? kLinkRightLeaf : 0u);
+}
+
+// The block-local climb of one thread (from its leaf `t`): nodes are made and
+// exchanged in shared memory only, so a level costs no global store that the
+// fences around the exchange would have to wait for; write_local writes them
+// out afterwards.  Returns true when the node in `c` waits for a split outside
+// the CTA (the thread goes on with it), false when this thread is done.
+template <typename K, int B>
+__device__ __forceinline__ bool climb_local(const BuildArgs<K>& A, Climb& c, BuildShared<K, B>& S,
+                                            uint32_t B0) {
+    const uint32_t n = A.n;
+    while (true) {
         const bool is_left = c.dr > c.dl;
-        const uint32_t gamma = is_left ? c.r : c.l - 1;
-        int qg = 0;
-        if (LOCAL) {
-            qg = (int)((long long)gamma - ((long long)B0 - 1));
-            local = local && qg >= 1 && qg <= B - 1 && S->local[qg];
-            c.local = local;
-        }
-        if (STOP && !local) {
-            // The parent split lies outside this CTA: leave it to the climb kernel.
-            A.frontier[atomicAdd(A.frontier_count, 1u)] = make_uint2(c.l, c.r);
-            return false;
-        }
-        // Past the stop test a split build's first kernel is always local;
-        // its nodes hold fewer than B bodies, so never take FP64.
-        const bool IN_LOCAL = LOCAL && (STOP || local);
-        uint32_t other;
-        if (IN_LOCAL) {
-            // Shared-memory exchange: this node's record (in shared memory)
-            // is released to the CTA before the slot changes hands.
-            __threadfence_block();
-            other = atomicExch(&S->bound[qg], is_left ? c.l : c.r);
-            if (other == kSentinel) return false;
-            __threadfence_block();
+        // boundary (relative) at which this node meets its sibling
+        const int q = (int)((is_left ? c.r : c.l - 1u) - B0) + 1;
+        if (q < 1 || q > B - 1 || !S.local[q]) return true;
+        __threadfence_block();  // this node's record before the exchange
+        const uint32_t other = atomicExch(&S.bound[q], is_left ? c.l : c.r);
+        if (other == kSentinel) return false;  // first to arrive: the sibling's thread goes on
+        __threadfence_block();
+        const uint32_t gamma = B0 + (uint32_t)q - 1u;
+        const uint32_t pl = is_left ? c.l : other, pr = is_left ? other : c.r;
+        const bool lleaf = pl == gamma, rleaf = pr == gamma + 1u;
+        float4 sm, sb, sq = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int k = is_left ? q : q - 1;  // the sibling: gamma + 1 or gamma
+        if (is_left ? rleaf : lleaf) {
+            sm = S.leaf[k];
+            sb = make_float4(sm.x, sm.y, sm.x, sm.y);
         } else {
-            // One acq_rel exchange releases this node's record and acquires
-            // the sibling's (release/acquire through bound[gamma]).
-            cuda::atomic_ref<uint32_t, cuda::thread_scope_device> slot(A.bound[gamma]);
-            other = slot.exchange(is_left ? c.l : c.r, cuda::memory_order_acq_rel);
-            if (other == kSentinel) return false;  // first to arrive: the sibling finishes the parent
-            slot.store(kSentinel, cuda::memory_order_relaxed);
+            sm = S.mom[k];
+            sb = S.box[k];
+            sq = S.quad[k];
         }
-        const uint32_t pl = is_left ? c.l : other;
-        const uint32_t pr = is_left ? other : c.r;
-        const uint32_t li = (pl == gamma) ? nm1 + gamma : gamma;
-        const uint32_t ri = (pr == gamma + 1) ? nm1 + gamma + 1 : gamma + 1;
-        const uint32_t sib = is_left ? ri : li;
-        const uint32_t sib_cnt = is_left ? (pr - gamma) : (gamma - pl + 1);
-        const uint32_t my_cnt = c.r - c.l + 1;
-        float4 s4, sb, sq = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (IN_LOCAL) {
-            // Sibling record from shared memory.
-            if (sib >= nm1) {
-                const int k = (int)(sib - nm1 - B0);
-                s4 = shared_leaf(S, k);
-                sb = make_float4(s4.x, s4.y, s4.x, s4.y);
-            } else {
-                const int k = (int)(sib - B0);
-                shared_rec(S, k, s4, sb, sq);
-            }
-        } else if (sib >= nm1) {
-            // Sibling record through L2 (written by another thread in this launch).
-            s4 = __ldcg(&A.node4[sib]);
-            sb = make_float4(s4.x, s4.y, s4.x, s4.y);
-        } else if (A.gnode) {
-            sb = __ldcg(&A.gnode[sib].box);
-            s4 = __ldcg(&A.gnode[sib].mom);
-            const float4 st = __ldcg(&A.gnode[sib].tail);
-            sq = make_float4(s4.w, st.x, st.y, 0.f);
-        } else {
-            s4 = __ldcg(&A.node4[sib]);
-            sb = __ldcg(&A.aabb[sib]);
-        }
+        // Parent's boundary deltas; its Karras index is its range end next to
+        // the larger one (the root's is 0, its first slot).
+        if (is_left) c.dr = S.d[(int)(pr - B0) + 1];
+        else c.dl = S.d[(int)(pl - B0)];
+        const uint32_t pidx = (c.dr > c.dl) ? pr : pl;
+        float tm, ncx, ncy;
+        join_centres(c.cm, c.cx, c.cy, sm.z, sm.x, sm.y, tm, ncx, ncy);
+        join_moments(c.cm, c.cx, c.cy, sm.z, sm.x, sm.y, ncx, ncy, sq, c.sxx, c.sxy, c.syy);
         c.lox = fminf(c.lox, sb.x);
         c.loy = fminf(c.loy, sb.y);
         c.hix = fmaxf(c.hix, sb.z);
         c.hiy = fmaxf(c.hiy, sb.w);
-        const uint32_t cnt = pr - pl + 1;
-        // Parent's boundary deltas and its own Karras index.
-        int dpl, dpr;
-        if (is_left) {
-            dpl = c.dl;
-            dpr = (IN_LOCAL) ? S->d[(int)(pr - B0 + 1)]
-                                   : ((pr == nm1) ? -1 : delta_at(A.keys, pr, pr + 1));
-        } else {
-            dpr = c.dr;
-            dpl = (IN_LOCAL) ? S->d[(int)(pl - B0)]
-                                   : ((pl == 0) ? -1 : delta_at(A.keys, pl - 1, pl));
-        }
-        const uint32_t pidx = (pl == 0 && pr == nm1) ? 0u : ((dpr > dpl) ? pr : pl);
-        float tm, ncx, ncy;
-        if (!STOP && A.fp64 && cnt >= kFp64MinBodies) {
-            double sm, smx, smy;
-            if (sib_cnt >= kFp64MinBodies) {
-                const double2 s0 = __ldcg(&A.big[2 * (size_t)sib]);
-                const double2 s1 = __ldcg(&A.big[2 * (size_t)sib + 1]);
-                sm = s0.x; smx = s0.y; smy = s1.x;
-            } else {
-                sm = (double)s4.z; smx = (double)s4.z * (double)s4.x; smy = (double)s4.z * (double)s4.y;
-            }
-            if (my_cnt < kFp64MinBodies) {
-                c.dm = (double)c.cm; c.dmx = (double)c.cm * (double)c.cx; c.dmy = (double)c.cm * (double)c.cy;
-            }
-            c.dm += sm;
-            c.dmx += smx;
-            c.dmy += smy;
-            tm = (float)c.dm;
-            const double inv = c.dm > 0.0 ? 1.0 / c.dm : 0.0;
-            ncx = (float)(c.dmx * inv);
-            ncy = (float)(c.dmy * inv);
-            A.big[2 * (size_t)pidx] = make_double2(c.dm, c.dmx);
-            A.big[2 * (size_t)pidx + 1] = make_double2(c.dmy, 0.0);
-        } else {
-            // (c_l m_l + c_r m_r) / (m_l + m_r).  Each sum is one IEEE addition
-            // of two terms, which is commutative, so this node's and the
-            // sibling's terms may be summed in either order with the same
-            // result; the split build's kernels (B >= 256) skip the left/right
-            // selects (16.8M-case build 5% faster), the fused build keeps
-            // them (measured 2.5% faster at 800k with them).
-            float ml = c.cm, mr = s4.z, clx = c.cx, cly = c.cy, crx = s4.x, cry = s4.y;
-            if (B < 256 && !is_left) {
-                ml = s4.z; clx = s4.x; cly = s4.y; mr = c.cm; crx = c.cx; cry = c.cy;
-            }
-            tm = __fadd_rn(ml, mr);
-            if (tm > 0.0f) {
-                const float inv = __frcp_rn(tm);
-                ncx = div_by(__fadd_rn(__fmul_rn(clx, ml), __fmul_rn(crx, mr)), tm, inv);
-                ncy = div_by(__fadd_rn(__fmul_rn(cly, ml), __fmul_rn(cry, mr)), tm, inv);
-            } else {
-                ncx = 0.0f;
-                ncy = 0.0f;
-            }
-        }
-        const float len = fmaxf(__fsub_rn(c.hix, c.lox), __fsub_rn(c.hiy, c.loy));
-        if (A.gnode) {
-            // Second moments about the parent COM:
-            // S = sum_c S_c + m_c d_c d_c^T, d_c = c_c - c_parent (leaves: S_c = 0),
-            // the two children's terms joined by one (commutative) addition;
-            // a and b are this node and its sibling, or (fused build) the
-            // left and the right child, as for the centre above.
-            float ma = c.cm, mb = s4.z, sax = c.sxx, say = c.sxy, saz = c.syy;
-            float sbx = sq.x, sby = sq.y, sbz = sq.z, pax = c.cx, pay = c.cy, pbx = s4.x, pby = s4.y;
-            if (B < 256 && !is_left) {
-                ma = s4.z; sax = sq.x; say = sq.y; saz = sq.z; pax = s4.x; pay = s4.y;
-                mb = c.cm; sbx = c.sxx; sby = c.sxy; sbz = c.syy; pbx = c.cx; pby = c.cy;
-            }
-            const float dax = __fsub_rn(pax, ncx), day = __fsub_rn(pay, ncy);
-            const float dbx = __fsub_rn(pbx, ncx), dby = __fsub_rn(pby, ncy);
-            const float madx = __fmul_rn(ma, dax), mady = __fmul_rn(ma, day);
-            const float mbdx = __fmul_rn(mb, dbx), mbdy = __fmul_rn(mb, dby);
-            c.sxx = __fadd_rn(__fmaf_rn(madx, dax, sax), __fmaf_rn(mbdx, dbx, sbx));
-            c.sxy = __fadd_rn(__fmaf_rn(madx, day, say), __fmaf_rn(mbdx, dby, sby));
-            c.syy = __fadd_rn(__fmaf_rn(mady, day, saz), __fmaf_rn(mbdy, dby, sbz));
-            GNode* const g = &A.gnode[pidx];
-            const uint32_t link = gamma | (li >= nm1 ? kLinkLeftLeaf : 0u) | (ri >= nm1 ? kLinkRightLeaf : 0u);
-            st_half(&g->mom, make_float4(ncx, ncy, tm, c.sxx),
-                    make_float4(c.sxy, c.syy, __uint_as_float(pl), __uint_as_float(cnt)));
-            st_half(&g->box, make_float4(c.lox, c.loy, c.hix, c.hiy),
-                    make_float4(ncx, ncy, __uint_as_float(link),
-                                __uint_as_float(pack_small(cnt, gamma - pl + 1u))));
-        }
-        if (A.groups) {
-            // Walk groups: maximal subtrees of <= gmax bodies.  A child is one
-            // when its parent is too big; the whole tree is one when n <= gmax.
-            if (cnt > A.gmax) {
-                const uint32_t lcnt = gamma - pl + 1, rcnt = pr - gamma;
-                if (lcnt <= A.gmax) A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(pl, lcnt);
-                if (rcnt <= A.gmax) A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(gamma + 1, rcnt);
-            } else if (pidx == 0) {
-                A.groups[atomicAdd(A.group_count, 1u)] = make_uint2(0u, n);
-            }
-        }
-        if (!A.gnode) {
-            // Reference layout (lbvh.wgsl:12-22, split into hot and cold
-            // arrays).  With the packed records it is derived on request
-            // (ref_layout_kernel): four scattered 8-16 B writes per node
-            // fewer in every step.
-            A.node4[pidx] = make_float4(ncx, ncy, tm, len);
-            A.aabb[pidx] = make_float4(c.lox, c.loy, c.hix, c.hiy);
-            A.children[pidx] = make_uint2(li, ri);
-            A.range[pidx] = make_uint2(pl, pr);
-        }
-        A.parent[li] = pidx;
-        A.parent[ri] = pidx;
-        if (pidx == 0) {
-            A.parent[0] = kSentinel;  // lbvh.wgsl:159-161
-            return false;
-        }
-        if (IN_LOCAL) {
-            // the new node is local: its record for the sibling that may meet it here
-            const int k = (int)(pidx - B0);
-            put_rec(S, k, make_float4(ncx, ncy, tm, 0.0f), make_float4(c.lox, c.loy, c.hix, c.hiy),
-                    make_float4(c.sxx, c.sxy, c.syy, 0.0f));
-        }
-        c.cm = tm; c.cx = ncx; c.cy = ncy;
+        c.cm = tm;
+        c.cx = ncx;
+        c.cy = ncy;
         c.l = pl;
         c.r = pr;
-        c.dl = dpl;
-        c.dr = dpr;
+        const int w = (int)(pidx - B0);
+        const uint32_t cnt = pr - pl + 1u;
+        S.mom[w] = make_float4(ncx, ncy, tm, __uint_as_float(make_link(gamma, lleaf, rleaf)));
+        S.box[w] = make_float4(c.lox, c.loy, c.hix, c.hiy);
+        S.quad[w] = make_float4(c.sxx, c.sxy, c.syy, __uint_as_float(cnt));
+        S.first[w] = (unsigned short)(pl - B0);
+        if (cnt == n) return false;  // the root
     }
-    return true;
 }
 
-// The whole climb of one thread.
-template <typename K, int B, bool LOCAL, bool STOP>
-__device__ __forceinline__ void climb(const BuildArgs<K>& A, Climb& c, BuildShared<K, B>* S,
-                                      uint32_t B0) {
-    while (climb_step<K, B, LOCAL, STOP>(A, c, S, B0)) {
+// One level of the climb with the device-scope protocol: returns false when
+// this thread is the first to arrive at the split (it stops; the sibling's
+// thread goes on) or has created the root, else true with `c` holding the
+// parent.
+template <typename K>
+__device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c) {
+    const uint32_t n = A.n, nm1 = n - 1;
+    const bool is_left = c.dr > c.dl;
+    const uint32_t gamma = is_left ? c.r : c.l - 1;
+    // One acq_rel exchange releases this node's record and acquires the
+    // sibling's (release/acquire through bound[gamma]).
+    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> slot(A.bound[gamma]);
+    const uint32_t other = slot.exchange(is_left ? c.l : c.r, cuda::memory_order_acq_rel);
+    if (other == kSentinel) return false;  // first to arrive: the sibling finishes the parent
+    slot.store(kSentinel, cuda::memory_order_relaxed);
+    const uint32_t pl = is_left ? c.l : other;
+    const uint32_t pr = is_left ? other : c.r;
+    const bool lleaf = pl == gamma, rleaf = pr == gamma + 1;
+    const uint32_t li = lleaf ? nm1 + gamma : gamma;
+    const uint32_t ri = rleaf ? nm1 + gamma + 1 : gamma + 1;
+    const uint32_t sib = is_left ? ri : li;
+    const uint32_t sib_cnt = is_left ? (pr - gamma) : (gamma - pl + 1);
+    const uint32_t my_cnt = c.r - c.l + 1;
+    // Sibling record through L2 (written by another thread in this launch).
+    float4 s4, sb, sq = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (sib >= nm1) {
+        s4 = __ldcg(&A.node4[sib]);
+        sb = make_float4(s4.x, s4.y, s4.x, s4.y);
+    } else if (A.gnode) {
+        sb = __ldcg(&A.gnode[sib].box);
+        s4 = __ldcg(&A.gnode[sib].mom);
+        const float4 st = __ldcg(&A.gnode[sib].tail);
+        sq = make_float4(s4.w, st.x, st.y, 0.f);
+    } else {
+        s4 = __ldcg(&A.node4[sib]);
+        sb = __ldcg(&A.aabb[sib]);
     }
+    c.lox = fminf(c.lox, sb.x);
+    c.loy = fminf(c.loy, sb.y);
+    c.hix = fmaxf(c.hix, sb.z);
+    c.hiy = fmaxf(c.hiy, sb.w);
+    const uint32_t cnt = pr - pl + 1;
+    // Parent's boundary deltas and its own Karras index.
+    if (is_left) c.dr = (pr == nm1) ? -1 : delta_at(A.keys, pr, pr + 1);
+    else c.dl = (pl == 0) ? -1 : delta_at(A.keys, pl - 1, pl);
+    const uint32_t pidx = (cnt == n) ? 0u : ((c.dr > c.dl) ? pr : pl);
+    float tm, ncx, ncy;
+    if (A.fp64 && cnt >= kFp64MinBodies) {
+        double sm, smx, smy;
+        if (sib_cnt >= kFp64MinBodies) {
+            const double2 s0 = __ldcg(&A.big[2 * (size_t)sib]);
+            const double2 s1 = __ldcg(&A.big[2 * (size_t)sib + 1]);
+            sm = s0.x; smx = s0.y; smy = s1.x;
+        } else {
+            sm = (double)s4.z; smx = (double)s4.z * (double)s4.x; smy = (double)s4.z * (double)s4.y;
+        }
+        if (my_cnt < kFp64MinBodies) {
+            c.dm = (double)c.cm; c.dmx = (double)c.cm * (double)c.cx; c.dmy = (double)c.cm * (double)c.cy;
+        }
+        c.dm += sm;
+        c.dmx += smx;
+        c.dmy += smy;
+        tm = (float)c.dm;
+        const double inv = c.dm > 0.0 ? 1.0 / c.dm : 0.0;
+        ncx = (float)(c.dmx * inv);
+        ncy = (float)(c.dmy * inv);
+        A.big[2 * (size_t)pidx] = make_double2(c.dm, c.dmx);
+        A.big[2 * (size_t)pidx + 1] = make_double2(c.dmy, 0.0);
+    } else {
+        join_centres(c.cm, c.cx, c.cy, s4.z, s4.x, s4.y, tm, ncx, ncy);
+    }
+    if (A.gnode)
+        join_moments(c.cm, c.cx, c.cy, s4.z, s4.x, s4.y, ncx, ncy, sq, c.sxx, c.sxy, c.syy);
+    emit_node(A, pidx, pl, cnt, make_link(gamma, lleaf, rleaf), ncx, ncy, tm,
+              make_float4(c.lox, c.loy, c.hix, c.hiy), c.sxx, c.sxy, c.syy);
+    c.cm = tm; c.cx = ncx; c.cy = ncy;
+    c.l = pl;
+    c.r = pr;
+    return cnt != n;
 }
 
 // Hierarchy build + fill, one thread per sorted slot.  SPLIT = false: the
@@ -538,34 +473,62 @@ build_fill_kernel(const BuildArgs<K> A) {
         }
         __syncthreads();
     }
-    if (i >= n) return;
-
-    const uint32_t body = __ldg(&A.ids[i]);
-    float m;
-    float2 p;
-    if (A.xm) {
-        const float4 r = __ldg(&A.xm[body]);
-        m = r.z;
-        p = make_float2(r.x, r.y);
-    } else {
-        m = __ldg(&A.mass[body]);
-        p = __ldg(&A.pos[body]);
-    }
-    A.node4[nm1 + i] = make_float4(p.x, p.y, m, 0.0f);  // leaf (lbvh.wgsl:179-187)
-    put_leaf(&S, t, make_float4(p.x, p.y, m, 0.0f));
+    S.quad[t] = make_float4(0.f, 0.f, 0.f, 0.f);  // no node yet
+    const bool active = i < n;
     Climb c;
-    c.l = i;
-    c.r = i;
-    // delta at the two boundaries of the current range (-1 outside [0, n-1]);
-    // a parent keeps one of them, so each level computes only one new delta.
-    c.dl = S.d[t];
-    c.dr = S.d[t + 1];
-    c.cm = m; c.cx = p.x; c.cy = p.y;
-    c.lox = p.x; c.loy = p.y; c.hix = p.x; c.hiy = p.y;
-    c.sxx = 0.0f; c.sxy = 0.0f; c.syy = 0.0f;
-    c.dm = 0.0; c.dmx = 0.0; c.dmy = 0.0;
-    c.local = true;
-    climb<K, B, true, SPLIT>(A, c, &S, B0);
+    if (active) {
+        const uint32_t body = __ldg(&A.ids[i]);
+        float4 r;
+        if (A.xm) {
+            r = __ldg(&A.xm[body]);
+        } else {
+            const float2 p = __ldg(&A.pos[body]);
+            r = make_float4(p.x, p.y, __ldg(&A.mass[body]), 0.0f);
+        }
+        r.w = 0.0f;
+        S.leaf[t] = r;
+        c.l = i;
+        c.r = i;
+        // delta at the two boundaries of the current range (-1 outside [0, n-1]);
+        // a parent keeps one of them, so each level computes only one new delta.
+        c.dl = S.d[t];
+        c.dr = S.d[t + 1];
+        c.cm = r.z; c.cx = r.x; c.cy = r.y;
+        c.lox = r.x; c.loy = r.y; c.hix = r.x; c.hiy = r.y;
+        c.sxx = 0.0f; c.sxy = 0.0f; c.syy = 0.0f;
+        c.dm = 0.0; c.dmx = 0.0; c.dmy = 0.0;
+    }
+    __syncthreads();
+    const bool on = active && climb_local<K, B>(A, c, S, B0);
+    __syncthreads();
+    // ---- write the CTA's leaves and local nodes, in order ------------------
+    if (active) A.node4[nm1 + i] = S.leaf[t];  // leaf (lbvh.wgsl:179-187)
+    {
+        const float4 quad = S.quad[t];
+        const uint32_t cnt = __float_as_uint(quad.w);
+        if (cnt != 0u) {
+            const float4 mom = S.mom[t];
+            emit_node(A, B0 + (uint32_t)t, B0 + (uint32_t)S.first[t], cnt, __float_as_uint(mom.w),
+                      mom.x, mom.y, mom.z, S.box[t], quad.x, quad.y, quad.z);
+        }
+    }
+    if (SPLIT) {
+        // nodes whose parent split lies outside this CTA: to the climb kernel
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, on);
+        if (m) {
+            uint32_t at = 0;
+            if (lane == __ffs(m) - 1) at = atomicAdd(A.frontier_count, (uint32_t)__popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, __ffs(m) - 1);
+            if (on) A.frontier[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] = make_uint2(c.l, c.r);
+        }
+        return;
+    }
+    // The CTA's records are written before any of its threads releases one of
+    // them (barrier, then the exchange's release at device scope).
+    __syncthreads();
+    if (on)
+        while (climb_step(A, c)) {
+        }
 }
 
 // Second kernel of the split build: one thread per frontier node (a node
@@ -590,7 +553,6 @@ build_climb_kernel(const BuildArgs<K> A) {
         c.dr = (c.r == nm1) ? -1 : delta_at(A.keys, c.r, c.r + 1);
         c.sxx = 0.0f; c.sxy = 0.0f; c.syy = 0.0f;
         c.dm = 0.0; c.dmx = 0.0; c.dmy = 0.0;
-        c.local = false;
         if (c.l == c.r) {
             const float4 leaf = A.node4[nm1 + c.l];
             c.cm = leaf.z; c.cx = leaf.x; c.cy = leaf.y;
@@ -611,7 +573,8 @@ build_climb_kernel(const BuildArgs<K> A) {
             c.cm = mom.z; c.cx = mom.x; c.cy = mom.y;
             c.lox = box.x; c.loy = box.y; c.hix = box.z; c.hiy = box.w;
         }
-        climb<K, kBuildBlockSplit, false, false>(A, c, nullptr, 0u);
+        while (climb_step(A, c)) {
+        }
     }
 }
 
