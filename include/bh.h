@@ -345,7 +345,7 @@ int bh_get_system_offsets(bh_sim* sim, uint32_t* offsets); /* num_systems + 1 en
  * GPU race, so serialise them.  Every call looks the scratch up with
  * cudaGetSymbolAddress in the current context.  Under CUDA's lazy module
  * loading the first call on a device may load this library's module, which
- * reserves the static array (about 11.5 MB) and may synchronise: a caller
+ * reserves the static array (about 31 MB) and may synchronise: a caller
  * that must not allocate while running makes one warm-up call at start-up,
  * before any stream capture.  Errors are reported through
  * bh_global_last_error(). */

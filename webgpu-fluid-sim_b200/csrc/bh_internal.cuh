@@ -31,7 +31,7 @@ constexpr uint32_t kErrStackOverflow = 1u << 1; // walk stack would have overflo
 constexpr uint32_t kErrTreeSpin = 1u << 2;
 // Failures after which the rest of a step has no valid input: the build and
 // the walk then skip their work for that step instead of consuming it.
-constexpr uint32_t kErrSkipMask = kErrLookbackSpin;
+constexpr uint32_t kErrSkipMask = kErrLookbackSpin | kErrTreeSpin;
 // Default spins of the sort's bounded look-back wait (several seconds).
 constexpr uint32_t kSpinCapDefault = 1u << 22;
 // Test hook: the second tile of the first sort pass waits on a predecessor
@@ -78,6 +78,17 @@ __device__ __forceinline__ void st_half(float4* p, const float4& a, const float4
                  "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
                  : "memory");
 }
+
+// Where the two children of a split meet in the hierarchy build (all ones
+// between steps): each swaps its record in, word by word, and the second gets
+// the first's out.  `side` (1 left, 2 right child) tells the two apart.
+//   w[0] {far range end, m, cx, cy}   w[1] {lox, loy, hix, side}
+//   w[2] {hiy, Sxx, Sxy, side}        w[3] {Syy, outer boundary's delta, 0, side}
+//   w[4..6] {FP64 sum of m, m x, m y, 0, side}: nodes of >= kFp64MinBodies
+struct __align__(16) MeetSlot {
+    uint4 w[7];
+};
+constexpr uint32_t kMeetSpins = 1u << 22;  // wait for a word under way (about a second)
 
 // Group acceptance test.  A node stands in for its bodies, as one multipole,
 // for a whole group when its size L and the distance d from the group's box
@@ -190,8 +201,7 @@ struct DeviceBuffers {
     uint32_t* parent = nullptr;  // 2n-1
     float4* aabb = nullptr;      // n-1 {min.x, min.y, max.x, max.y}
     uint2* range = nullptr;      // n-1 {first slot, last slot}
-    double2* big = nullptr;      // 2(n-1) FP64 {mass, mass*x}, {mass*y, 0} for big nodes
-    uint32_t* bound = nullptr;   // n-1 exchange slots, kSentinel between steps
+    MeetSlot* slots = nullptr;   // n-1, one per split: all ones between steps
     GNode* gnode = nullptr;      // n-1 packed records (group walk only; else null)
     uint2* groups = nullptr;     // n {first slot, count}: maximal subtrees of <= G bodies (group walk)
     uint32_t group_max = 0;      // G = 32 x bodies per lane (0: no groups)
@@ -248,15 +258,14 @@ uint32_t sort_tiles(uint32_t n);  // tiles of the sort of n keys
 // tree.cu
 void launch_build_fill(const DeviceBuffers& b, int fp64_levels, cudaStream_t s);
 // Bodies from which the build runs as two kernels (local phase + frontier climb).
-// Measured crossover (tree stage, B200): 0.8M fused 0.137 / split 0.151 ms, 1.5M
-// equal (0.211), 3M fused 0.371 / split 0.342, 4.2M 0.556 / 0.470.
+// Measured crossover (tree stage, B200): 0.8M fused 0.093 / split 0.105 ms, 1.5M
+// equal (0.153), 2.2M 0.228 / 0.225, 4.2M 0.404 / 0.374.
 #ifndef BH_SPLIT_BUILD_MIN
 #define BH_SPLIT_BUILD_MIN (1u << 21)
 #endif
 constexpr uint32_t kSplitBuildMin = BH_SPLIT_BUILD_MIN;
 bool split_build(uint32_t n, uint32_t debug_flags);
 void launch_ref_layout(const DeviceBuffers& b, cudaStream_t s);  // group walk: node4/aabb/children/range on request
-void init_bound(const DeviceBuffers& b, cudaStream_t s);
 // walk.cu
 void launch_walk(const DeviceBuffers& b, const WalkParams& p, int block, cudaStream_t s);
 // walk_group.cu

@@ -342,8 +342,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     size_t o_codes = c.take<uint8_t>(nb * kb), o_codes2 = c.take<uint8_t>(nb * kb);
     size_t o_ids = c.take<uint32_t>(nb), o_ids2 = c.take<uint32_t>(nb);
     size_t o_node4 = c.take<float4>(nn), o_child = c.take<uint2>(ni), o_parent = c.take<uint32_t>(nn);
-    size_t o_aabb = c.take<float4>(ni), o_range = c.take<uint2>(ni), o_big = c.take<double2>(2 * ni);
-    size_t o_bound = c.take<uint32_t>(ni);
+    size_t o_aabb = c.take<float4>(ni), o_range = c.take<uint2>(ni);
     size_t o_front = c.take<uint2>(nb);
     const bool group = s->cfg.walk_mode == BH_WALK_GROUP;
     size_t o_gnode = group ? c.take<bh::GNode>(ni) : 0;
@@ -358,6 +357,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     size_t o_stpos = c.take<float2>(nb), o_stmass = c.take<float>(nb), o_stvel = c.take<float2>(nb);
     size_t o_smass = c.take<float>(nb);
     size_t o_spos = c.take<float2>(nb), o_svel = c.take<float2>(nb);
+    size_t o_slots = c.take<bh::MeetSlot>(ni);  // last: starts at all ones, the rest at zero
     void* arena = nullptr;
     cudaError_t e = cudaMalloc(&arena, c.off);
     if (e != cudaSuccess) {
@@ -386,8 +386,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     b.parent = (uint32_t*)(a + o_parent);
     b.aabb = (float4*)(a + o_aabb);
     b.range = (uint2*)(a + o_range);
-    b.big = (double2*)(a + o_big);
-    b.bound = (uint32_t*)(a + o_bound);
+    b.slots = (bh::MeetSlot*)(a + o_slots);
     b.frontier = (uint2*)(a + o_front);
     b.gnode = group ? (bh::GNode*)(a + o_gnode) : nullptr;
     b.groups = group ? (uint2*)(a + o_groups) : nullptr;
@@ -408,8 +407,8 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     s->snap_mass = (float*)(a + o_smass);
     s->snap_pos = (float2*)(a + o_spos);
     s->snap_vel = (float2*)(a + o_svel);
-    BH_CUDA(s, cudaMemsetAsync(arena, 0, c.off, s->stream));
-    BH_CUDA(s, cudaMemsetAsync(b.bound, 0xFF, sizeof(uint32_t) * ni, s->stream));
+    BH_CUDA(s, cudaMemsetAsync(arena, 0, o_slots, s->stream));
+    BH_CUDA(s, cudaMemsetAsync(b.slots, 0xFF, c.off - o_slots, s->stream));
     if (E) {
         // offsets and per-body system ids (systems are contiguous)
         std::vector<uint32_t> off(E + 1, 0), bsys(nb, 0);
@@ -614,8 +613,9 @@ static int check_device_errors(bh_sim* s) {
     if (e & bh::kErrTreeSpin) msg += " tree build gave up waiting;";
     if (e & bh::kErrGroupStack) msg += " group-walk stack full;";
     if (e & bh::kErrShardCapacity) msg += " shard chunk too small for its updated bodies;";
-    // Restore the build's exchange slots so the next step starts clean.
-    if (s->b.n > 1) BH_CUDA(s, cudaMemsetAsync(s->b.bound, 0xFF, sizeof(uint32_t) * (s->b.n - 1), s->stream));
+    // Restore the build's meeting slots so the next step starts clean.
+    if (s->b.n > 1)
+        BH_CUDA(s, cudaMemsetAsync(s->b.slots, 0xFF, sizeof(bh::MeetSlot) * ((size_t)s->b.n - 1), s->stream));
     return fail(s, BH_ERR_DEVICE_CHECK, msg);
 }
 

@@ -27,10 +27,6 @@ cudaError_t build_init_attributes() {
     return set_build_attributes<uint64_t, true>();
 }
 
-void init_bound(const DeviceBuffers& b, cudaStream_t s) {
-    if (b.n > 1) cudaMemsetAsync(b.bound, 0xFF, sizeof(uint32_t) * (b.n - 1), s);
-}
-
 template <typename K>
 static void launch_typed(const DeviceBuffers& b, int fp64_levels, cudaStream_t s) {
     BuildArgs<K> a;
@@ -43,8 +39,7 @@ static void launch_typed(const DeviceBuffers& b, int fp64_levels, cudaStream_t s
     a.parent = b.parent;
     a.aabb = b.aabb;
     a.range = b.range;
-    a.big = b.big;
-    a.bound = b.bound;
+    a.slots = b.slots;
     a.n = b.n;
     a.fp64 = fp64_levels;
     a.gnode = b.gnode;

@@ -19,12 +19,12 @@
 // (lbvh.wgsl:141-152).  Computing those indices here gives the same
 // left/right/parent arrays as the reference's top-down build, bit for bit.
 //
-// Synchronisation: the two children of a split gamma meet at bound[gamma] with
-// an atomic exchange of their far range ends; the first arriver stops.  The
-// exchange is acq_rel at device scope: it releases the node record this
-// thread wrote and acquires the sibling's, which the second arriver then reads
-// through L2 (__ldcg), so no stale data is ever combined.  There are no spins.
-// bound[] holds kSentinel between steps: the second arriver restores it.
+// Synchronisation: the two children of a split gamma meet at its slot with
+// atomic exchanges of their records; the first arriver (by the range ends'
+// word) stops, the second has the other's record from the same exchanges.
+// No other data passes between threads, so there are no fences.  A word of
+// the sibling that has not landed yet is awaited (bounded; its exchange was
+// issued before).  The second arriver empties the slot (all ones between steps).
 //
 // Two phases per climb.  A CTA owns B consecutive slots (128 in the fused
 // build, 512 in the split build's local phase).  A node whose
@@ -95,8 +95,7 @@ struct BuildArgs {
     uint32_t* parent;
     float4* aabb;
     uint2* range;
-    double2* big;
-    uint32_t* bound;
+    MeetSlot* slots;
     uint32_t n;
     int fp64;
     GNode* gnode;
@@ -111,18 +110,19 @@ struct BuildArgs {
     // one gather per slot instead of a position and a mass
     const float4* xm = nullptr;
     // The step's device error word: when an earlier stage of the step failed
-    // (kErrSkipMask), the build does nothing.  Null: no such check.
-    const uint32_t* err = nullptr;
+    // (kErrSkipMask), the build does nothing; a bounded wait that gives up sets
+    // kErrTreeSpin.  Null: no such check.
+    uint32_t* err = nullptr;
 };
 
 // One thread per sorted slot climbs from its leaf; the lanes of a warp start
 // at adjacent leaves, so the low levels they create are adjacent in memory.
 // (A persistent variant that hands each finished lane a new leaf measured
 // slower at 16M bodies: its lanes drift apart and its node writes scatter.)
-// Slots per CTA (measured, B200): the fused build is fastest with small CTAs
-// (800k bodies: 128 -> 0.137 ms, 256 -> 0.140, 512 -> 0.150), the local phase
-// of the split build with large ones (16.8M: 128 -> 2.11 ms, 256 -> 1.83,
-// 512 -> 1.72).  The frontier climb keeps 256 threads per CTA.
+// Slots per CTA (tree stage, B200): the fused build, 64 / 128 / 256: 800k bodies
+// 102 / 93 / 96 us, 1.5M 170 / 154 / 160, 16k and fewer equal; the split
+// build's local phase takes large ones (16.8M, 256 / 512: 1.52 / 1.43 ms; 4.2M
+// 356 / 374 us).  The frontier climb keeps 256 threads per CTA.
 #ifndef BH_BUILD_BLOCK_FUSED
 #define BH_BUILD_BLOCK_FUSED 128
 #endif
@@ -134,13 +134,9 @@ constexpr int kBuildBlockSplit = BH_BUILD_BLOCK_SPLIT;
 constexpr int kClimbBlock = 256;
 template <bool SPLIT>
 constexpr int build_block() { return SPLIT ? kBuildBlockSplit : kBuildBlockFused; }
-// Resident CTAs per SM the launch bounds ask for.  The split build's local
-// phase issues in only ~60% of its cycles with 2 CTAs of 512 threads (47
-// registers); asking for 3 gives 40 registers with 16 B of spills and a
-// faster build (16.8M bodies: 1.86 -> 1.71 ms).  The fused build keeps the
-// compiler's choice (0: no minimum): 10 or 12 resident CTAs of 128 threads
-// (42-51 registers, spills) made it slower at 800k bodies (0.137 -> 0.143 /
-// 0.150 ms).
+// Resident CTAs per SM the launch bounds ask for: 3 for the split build's local
+// phase (39 registers, no spills; 4: 16.8M bodies 1.53 against 1.43 ms), the
+// compiler's choice (0) for the fused build.
 #ifndef BH_BUILD_MIN_BLOCKS_SPLIT
 #define BH_BUILD_MIN_BLOCKS_SPLIT 3
 #endif
@@ -307,80 +303,136 @@ __device__ __forceinline__ bool climb_local(const BuildArgs<K>& A, Climb& c, Bui
     }
 }
 
-// One level of the climb with the device-scope protocol: returns false when
-// this thread is the first to arrive at the split (it stops; the sibling's
-// thread goes on) or has created the root, else true with `c` holding the
-// parent.
+// 128-bit relaxed accesses at device scope (single-copy atomic).
+__device__ __forceinline__ uint4 exch128(uint4* p, uint4 v) {
+    uint4 r;
+    asm volatile(
+        "{\n .reg .b128 a, b;\n .reg .b64 l, h;\n mov.b64 l, {%5, %6};\n mov.b64 h, {%7, %8};\n"
+        " mov.b128 a, {l, h};\n atom.relaxed.gpu.global.exch.b128 b, [%4], a;\n"
+        " mov.b128 {l, h}, b;\n mov.b64 {%0, %1}, l;\n mov.b64 {%2, %3}, h;\n}"
+        : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+        : "l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+        : "memory");
+    return r;
+}
+__device__ __forceinline__ uint4 ld128(const uint4* p) {
+    uint4 r;
+    asm volatile(
+        "{\n .reg .b128 b;\n .reg .b64 l, h;\n ld.relaxed.gpu.global.b128 b, [%4];\n"
+        " mov.b128 {l, h}, b;\n mov.b64 {%0, %1}, l;\n mov.b64 {%2, %3}, h;\n}"
+        : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+        : "l"(p)
+        : "memory");
+    return r;
+}
+__device__ __forceinline__ void clear128(uint4* p) {
+    asm volatile(
+        "{\n .reg .b128 a;\n .reg .b64 l;\n mov.b64 l, -1;\n mov.b128 a, {l, l};\n"
+        " st.relaxed.gpu.global.b128 [%0], a;\n}" ::"l"(p)
+        : "memory");
+}
+
+// The sibling's word k of a split: `got` when this thread's exchange returned
+// it, else it is on its way (the sibling's exchanges were all issued before
+// the one that made this thread the second) and overwrites this thread's own.
+// Bounded; false when the wait gives up.
+__device__ __forceinline__ bool sibling_word(uint4& got, const uint4* p, uint32_t side) {
+    for (uint32_t spins = 0; got.w != side; ++spins) {
+        if (spins > kMeetSpins) return false;
+        if (spins > 64) __nanosleep(64);
+        got = ld128(p);
+    }
+    return true;
+}
+
+// One level of the climb at device scope: returns false when this thread is
+// the first to arrive at the split (it stops; the sibling's thread goes on)
+// or has created the root, else true with `c` holding the parent.  The two
+// children swap their whole records through the split's slot: every word is
+// one 128-bit exchange, all of them in flight together, so a level is one
+// round trip to the L2 and its arithmetic.  (An acq_rel exchange of the range
+// ends, then the sibling's record and the boundary's keys, is three in a row:
+// 3,000-3,300 cycles a level, 13 levels at 2k bodies, 27 at 800k, about 1,300
+// now.  Tree stage: 2k bodies 32 -> 20 us, 16k 39 -> 25, 100k 48 -> 31, 800k
+// 120 -> 93, 16.8M, bound by its local phase, 1.43 ms either way.)
 template <typename K>
 __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c) {
-    const uint32_t n = A.n, nm1 = n - 1;
+    const uint32_t n = A.n;
     const bool is_left = c.dr > c.dl;
     const uint32_t gamma = is_left ? c.r : c.l - 1;
-    // One acq_rel exchange releases this node's record and acquires the
-    // sibling's (release/acquire through bound[gamma]).
-    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> slot(A.bound[gamma]);
-    const uint32_t other = slot.exchange(is_left ? c.l : c.r, cuda::memory_order_acq_rel);
-    if (other == kSentinel) return false;  // first to arrive: the sibling finishes the parent
-    slot.store(kSentinel, cuda::memory_order_relaxed);
+    const uint32_t side = is_left ? 1u : 2u, other_side = 3u - side;
+    uint4* const w = A.slots[gamma].w;
+    const uint32_t my_cnt = c.r - c.l + 1;
+    const bool big = A.fp64 && my_cnt >= kFp64MinBodies;  // carries FP64 sums
+    auto bits = [](float v) { return __float_as_uint(v); };
+    auto word64 = [&](double v) {
+        return make_uint4((uint32_t)__double2loint(v), (uint32_t)__double2hiint(v), 0u, side);
+    };
+    uint4 o4 = make_uint4(0u, 0u, 0u, 0u), o5 = o4, o6 = o4;
+    if (big) {
+        o4 = exch128(w + 4, word64(c.dm));
+        o5 = exch128(w + 5, word64(c.dmx));
+        o6 = exch128(w + 6, word64(c.dmy));
+    }
+    uint4 o1 = exch128(w + 1, make_uint4(bits(c.lox), bits(c.loy), bits(c.hix), side));
+    uint4 o2 = exch128(w + 2, make_uint4(bits(c.hiy), bits(c.sxx), bits(c.sxy), side));
+    uint4 o3 = exch128(w + 3, make_uint4(bits(c.syy), (uint32_t)(is_left ? c.dl : c.dr), 0u, side));
+    const uint4 o0 = exch128(w, make_uint4(is_left ? c.l : c.r, bits(c.cm), bits(c.cx), bits(c.cy)));
+    if (o0.x == kSentinel) return false;  // first to arrive: the sibling finishes the parent
+    const uint32_t other = o0.x;
     const uint32_t pl = is_left ? c.l : other;
     const uint32_t pr = is_left ? other : c.r;
-    const bool lleaf = pl == gamma, rleaf = pr == gamma + 1;
-    const uint32_t li = lleaf ? nm1 + gamma : gamma;
-    const uint32_t ri = rleaf ? nm1 + gamma + 1 : gamma + 1;
-    const uint32_t sib = is_left ? ri : li;
     const uint32_t sib_cnt = is_left ? (pr - gamma) : (gamma - pl + 1);
-    const uint32_t my_cnt = c.r - c.l + 1;
-    // Sibling record through L2 (written by another thread in this launch).
-    float4 s4, sb, sq = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (sib >= nm1) {
-        s4 = __ldcg(&A.node4[sib]);
-        sb = make_float4(s4.x, s4.y, s4.x, s4.y);
-    } else if (A.gnode) {
-        sb = __ldcg(&A.gnode[sib].box);
-        s4 = __ldcg(&A.gnode[sib].mom);
-        const float4 st = __ldcg(&A.gnode[sib].tail);
-        sq = make_float4(s4.w, st.x, st.y, 0.f);
-    } else {
-        s4 = __ldcg(&A.node4[sib]);
-        sb = __ldcg(&A.aabb[sib]);
+    const bool sib_big = A.fp64 && sib_cnt >= kFp64MinBodies;
+    bool ok = sibling_word(o1, w + 1, other_side) && sibling_word(o2, w + 2, other_side) &&
+              sibling_word(o3, w + 3, other_side);
+    if (sib_big)
+        ok = ok && sibling_word(o4, w + 4, other_side) && sibling_word(o5, w + 5, other_side) &&
+             sibling_word(o6, w + 6, other_side);
+    if (!ok) {
+        if (A.err) atomicOr(A.err, kErrTreeSpin);
+        return false;
     }
-    c.lox = fminf(c.lox, sb.x);
-    c.loy = fminf(c.loy, sb.y);
-    c.hix = fmaxf(c.hix, sb.z);
-    c.hiy = fmaxf(c.hiy, sb.w);
+    // The slot is empty again for the next step (both children are done with it).
+    clear128(w);
+    clear128(w + 1);
+    clear128(w + 2);
+    clear128(w + 3);
+    if (big || sib_big) {
+        clear128(w + 4);
+        clear128(w + 5);
+        clear128(w + 6);
+    }
+    const float sm = __uint_as_float(o0.y), sx = __uint_as_float(o0.z), sy = __uint_as_float(o0.w);
+    c.lox = fminf(c.lox, __uint_as_float(o1.x));
+    c.loy = fminf(c.loy, __uint_as_float(o1.y));
+    c.hix = fmaxf(c.hix, __uint_as_float(o1.z));
+    c.hiy = fmaxf(c.hiy, __uint_as_float(o2.x));
+    const float4 sq = make_float4(__uint_as_float(o2.y), __uint_as_float(o2.z), __uint_as_float(o3.x), 0.f);
     const uint32_t cnt = pr - pl + 1;
-    // Parent's boundary deltas and its own Karras index.
-    if (is_left) c.dr = (pr == nm1) ? -1 : delta_at(A.keys, pr, pr + 1);
-    else c.dl = (pl == 0) ? -1 : delta_at(A.keys, pl - 1, pl);
+    // Parent's boundary deltas (the sibling's outer one is the parent's) and
+    // its own Karras index.
+    if (is_left) c.dr = (int)o3.y;
+    else c.dl = (int)o3.y;
     const uint32_t pidx = (cnt == n) ? 0u : ((c.dr > c.dl) ? pr : pl);
     float tm, ncx, ncy;
     if (A.fp64 && cnt >= kFp64MinBodies) {
-        double sm, smx, smy;
-        if (sib_cnt >= kFp64MinBodies) {
-            const double2 s0 = __ldcg(&A.big[2 * (size_t)sib]);
-            const double2 s1 = __ldcg(&A.big[2 * (size_t)sib + 1]);
-            sm = s0.x; smx = s0.y; smy = s1.x;
-        } else {
-            sm = (double)s4.z; smx = (double)s4.z * (double)s4.x; smy = (double)s4.z * (double)s4.y;
-        }
-        if (my_cnt < kFp64MinBodies) {
+        auto sum64 = [](const uint4& o) { return __hiloint2double((int)o.y, (int)o.x); };
+        if (!big) {
             c.dm = (double)c.cm; c.dmx = (double)c.cm * (double)c.cx; c.dmy = (double)c.cm * (double)c.cy;
         }
-        c.dm += sm;
-        c.dmx += smx;
-        c.dmy += smy;
+        c.dm += sib_big ? sum64(o4) : (double)sm;
+        c.dmx += sib_big ? sum64(o5) : (double)sm * (double)sx;
+        c.dmy += sib_big ? sum64(o6) : (double)sm * (double)sy;
         tm = (float)c.dm;
         const double inv = c.dm > 0.0 ? 1.0 / c.dm : 0.0;
         ncx = (float)(c.dmx * inv);
         ncy = (float)(c.dmy * inv);
-        A.big[2 * (size_t)pidx] = make_double2(c.dm, c.dmx);
-        A.big[2 * (size_t)pidx + 1] = make_double2(c.dmy, 0.0);
     } else {
-        join_centres(c.cm, c.cx, c.cy, s4.z, s4.x, s4.y, tm, ncx, ncy);
+        join_centres(c.cm, c.cx, c.cy, sm, sx, sy, tm, ncx, ncy);
     }
-    if (A.gnode)
-        join_moments(c.cm, c.cx, c.cy, s4.z, s4.x, s4.y, ncx, ncy, sq, c.sxx, c.sxy, c.syy);
-    emit_node(A, pidx, pl, cnt, make_link(gamma, lleaf, rleaf), ncx, ncy, tm,
+    if (A.gnode) join_moments(c.cm, c.cx, c.cy, sm, sx, sy, ncx, ncy, sq, c.sxx, c.sxy, c.syy);
+    emit_node(A, pidx, pl, cnt, make_link(gamma, pl == gamma, pr == gamma + 1), ncx, ncy, tm,
               make_float4(c.lox, c.loy, c.hix, c.hiy), c.sxx, c.sxy, c.syy);
     c.cm = tm; c.cx = ncx; c.cy = ncy;
     c.l = pl;
@@ -393,10 +445,10 @@ __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c) {
 // phase; threads that reach a split outside their CTA list their node in the
 // frontier and exit, and build_climb_kernel finishes the tree.  A CTA of the
 // fused build stays resident while one or two of its threads climb the
-// device-scope levels (a few L2 round trips each); the split build frees it
-// at the end of its local phase and climbs all frontier nodes side by side,
-// which pays off from a few million bodies up (measured: 2.14 -> 1.87 ms at
-// 16.8M bodies; at 800k the extra launch costs about as much as it saves).
+// device-scope levels; the split build frees it at the end of its local phase
+// and climbs all frontier nodes side by side, which pays off from a few
+// million bodies up (fused / split: 800k 93 / 105 us, 1.5M 154 / 152, 4.2M
+// 404 / 374, 16.8M 1.51 / 1.43 ms).
 // (Climbing the local phase in CTA-wide rounds that pack the remaining
 // nodes into the lowest warps measured slower.  Nor do the random leaf
 // gathers set the pace: with the bodies uploaded in the previous step's
@@ -523,9 +575,6 @@ build_fill_kernel(const BuildArgs<K> A) {
         }
         return;
     }
-    // The CTA's records are written before any of its threads releases one of
-    // them (barrier, then the exchange's release at device scope).
-    __syncthreads();
     if (on)
         while (climb_step(A, c)) {
         }

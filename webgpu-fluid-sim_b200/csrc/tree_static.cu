@@ -11,7 +11,7 @@
 // and the per-node slot ranges -- in the file-scope array below.
 //
 // Limits and sharing rules:
-//  - at most kStaticMaxBodies bodies per call (the array is ~11.5 MB and
+//  - at most kStaticMaxBodies bodies per call (the array is ~31 MB and
 //    every GPU that loads the library holds it until the process exits);
 //  - all calls share the one array, which keeps the last call's contents;
 //    each call resets the exchange slots it uses before its launch, and the
@@ -39,10 +39,9 @@ constexpr uint32_t kStaticMaxBodies = 262144;
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t v) { return (v + kAlign - 1) & ~(kAlign - 1); }
 // Layout inside the array (internal nodes: kStaticMaxBodies - 1).
-constexpr size_t kBoundOff = 0;
-constexpr size_t kRangeOff = align_up(kBoundOff + sizeof(uint32_t) * (kStaticMaxBodies - 1));
-constexpr size_t kBigOff = align_up(kRangeOff + sizeof(uint2) * (kStaticMaxBodies - 1));
-constexpr size_t kScratchBytes = align_up(kBigOff + 2 * sizeof(double2) * (kStaticMaxBodies - 1));
+constexpr size_t kSlotsOff = 0;
+constexpr size_t kRangeOff = align_up(kSlotsOff + sizeof(MeetSlot) * (kStaticMaxBodies - 1));
+constexpr size_t kScratchBytes = align_up(kRangeOff + sizeof(uint2) * (kStaticMaxBodies - 1));
 
 static __device__ __align__(256) unsigned char g_tree_scratch[kScratchBytes];
 
@@ -60,8 +59,8 @@ static cudaError_t scratch_address(unsigned char** out) {
 template <typename K>
 static void launch_static(const void* codes, const uint32_t* ids, const float* mass,
                           const float* pos, uint32_t n, float* node4, uint32_t* children,
-                          uint32_t* parent, float* aabb, uint2* range, double2* big,
-                          uint32_t* bound, int fp64, cudaStream_t s) {
+                          uint32_t* parent, float* aabb, uint2* range, MeetSlot* slots,
+                          int fp64, cudaStream_t s) {
     BuildArgs<K> a;
     a.keys = static_cast<const K*>(codes);
     a.ids = ids;
@@ -72,8 +71,7 @@ static void launch_static(const void* codes, const uint32_t* ids, const float* m
     a.parent = parent;
     a.aabb = reinterpret_cast<float4*>(aabb);
     a.range = range;
-    a.big = big;
-    a.bound = bound;
+    a.slots = slots;
     a.n = n;
     a.fp64 = fp64;
     a.gnode = nullptr;
@@ -113,24 +111,23 @@ extern "C" int bh_build_hierarchy_static(const void* sorted_codes, int32_t morto
     if (e != cudaSuccess)
         return static_fail(BH_ERR_CUDA, std::string("cudaGetSymbolAddress(static tree scratch): ") +
                                             cudaGetErrorString(e));
-    uint32_t* bound = reinterpret_cast<uint32_t*>(base + kBoundOff);
+    MeetSlot* slots = reinterpret_cast<MeetSlot*>(base + kSlotsOff);
     uint2* range = reinterpret_cast<uint2*>(base + kRangeOff);
-    double2* big = reinterpret_cast<double2*>(base + kBigOff);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // The exchange slots must start at kSentinel (the previous call may have
+    // The meeting slots must start at all ones (the previous call may have
     // been cut short by an error).
     if (n > 1) {
-        e = cudaMemsetAsync(bound, 0xFF, sizeof(uint32_t) * (n - 1), s);
+        e = cudaMemsetAsync(slots, 0xFF, sizeof(MeetSlot) * (size_t)(n - 1), s);
         if (e != cudaSuccess)
-            return static_fail(BH_ERR_CUDA, std::string("cudaMemsetAsync(static exchange slots): ") +
+            return static_fail(BH_ERR_CUDA, std::string("cudaMemsetAsync(static meeting slots): ") +
                                                 cudaGetErrorString(e));
     }
     if (morton_bits == 64)
         launch_static<uint64_t>(sorted_codes, sorted_ids, mass, pos, n, node4, node_children,
-                                node_parent, node_aabb, range, big, bound, fp64_levels, s);
+                                node_parent, node_aabb, range, slots, fp64_levels, s);
     else
         launch_static<uint32_t>(sorted_codes, sorted_ids, mass, pos, n, node4, node_children,
-                                node_parent, node_aabb, range, big, bound, fp64_levels, s);
+                                node_parent, node_aabb, range, slots, fp64_levels, s);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return static_fail(BH_ERR_CUDA, std::string("build_fill_kernel launch: ") + cudaGetErrorString(e));
