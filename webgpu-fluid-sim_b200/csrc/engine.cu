@@ -337,27 +337,32 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     const size_t nn = n ? 2 * (size_t)n - 1 : 1, ni = n > 1 ? (size_t)n - 1 : 1, nb = n ? n : 1;
     const uint32_t tiles = bh::sort_tiles(n);
     Carver c;
+    const bool group = s->cfg.walk_mode == BH_WALK_GROUP;
+    // ---- starts at zero: what a caller can read before the first step ------
     size_t o_mass = c.take<float>(nb), o_pos = c.take<float2>(nb), o_vel = c.take<float2>(nb);
-    size_t o_acc = c.take<float2>(nb), o_rad = c.take<float>(nb), o_xm = c.take<float4>(nb);
-    size_t o_codes = c.take<uint8_t>(nb * kb), o_codes2 = c.take<uint8_t>(nb * kb);
-    size_t o_ids = c.take<uint32_t>(nb), o_ids2 = c.take<uint32_t>(nb);
+    size_t o_acc = c.take<float2>(nb), o_rad = c.take<float>(nb);
+    size_t o_codes = c.take<uint8_t>(nb * kb), o_ids = c.take<uint32_t>(nb);
     size_t o_node4 = c.take<float4>(nn), o_child = c.take<uint2>(ni), o_parent = c.take<uint32_t>(nn);
     size_t o_aabb = c.take<float4>(ni), o_range = c.take<uint2>(ni);
-    size_t o_front = c.take<uint2>(nb);
-    const bool group = s->cfg.walk_mode == BH_WALK_GROUP;
     size_t o_gnode = group ? c.take<bh::GNode>(ni) : 0;
-    size_t o_groups = group ? c.take<uint2>(nb) : 0;
     size_t o_scr = c.take<bh::StepScratch>(1);
-    size_t o_status = c.take<uint32_t>((size_t)kb * (tiles ? tiles : 1) * bh::kRadix);
     size_t o_err = c.take<uint32_t>(1);
     size_t o_diag = c.take<double>(8);
     size_t o_soff = E ? c.take<uint32_t>(E + 1) : 0, o_bsys = E ? c.take<uint32_t>(nb) : 0;
     size_t o_sbox = E ? c.take<uint32_t>(4 * (size_t)E) : 0;
+    const size_t zero_end = c.off;
+    // ---- written before it is read in every step ----------------------------
+    size_t o_xm = c.take<float4>(nb);
+    size_t o_codes2 = c.take<uint8_t>(nb * kb), o_ids2 = c.take<uint32_t>(nb);
+    size_t o_front = c.take<uint2>(nb);
+    size_t o_groups = group ? c.take<uint2>(nb) : 0;
+    size_t o_status = c.take<uint32_t>((size_t)kb * (tiles ? tiles : 1) * bh::kRadix);
     // staged uploads and the asynchronous download's snapshot
     size_t o_stpos = c.take<float2>(nb), o_stmass = c.take<float>(nb), o_stvel = c.take<float2>(nb);
     size_t o_smass = c.take<float>(nb);
     size_t o_spos = c.take<float2>(nb), o_svel = c.take<float2>(nb);
-    size_t o_slots = c.take<bh::MeetSlot>(ni);  // last: starts at all ones, the rest at zero
+    // ---- starts at all ones ---------------------------------------------------
+    size_t o_slots = c.take<bh::MeetSlot>(ni);
     void* arena = nullptr;
     cudaError_t e = cudaMalloc(&arena, c.off);
     if (e != cudaSuccess) {
@@ -407,7 +412,7 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
     s->snap_mass = (float*)(a + o_smass);
     s->snap_pos = (float2*)(a + o_spos);
     s->snap_vel = (float2*)(a + o_svel);
-    BH_CUDA(s, cudaMemsetAsync(arena, 0, o_slots, s->stream));
+    BH_CUDA(s, cudaMemsetAsync(arena, 0, zero_end, s->stream));
     BH_CUDA(s, cudaMemsetAsync(b.slots, 0xFF, c.off - o_slots, s->stream));
     if (E) {
         // offsets and per-body system ids (systems are contiguous)
