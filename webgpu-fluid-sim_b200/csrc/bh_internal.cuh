@@ -113,6 +113,32 @@ __device__ __forceinline__ bool step_failed(const uint32_t* err) {
     return err && (__ldcg(err) & kErrSkipMask) != 0u;
 }
 
+// Programmatic dependent launch: a kernel of the step may be launched while the
+// one before it drains; it waits here, before it touches memory, until that one
+// is complete.  (Every kernel of the chain waits first, so completion is
+// transitive.)  Step, plain / chained: 2k bodies 48.7 / 46.6 us, 16k 74.4 /
+// 71.6, 50k 70.9 / 68.5, 800k equal.  Nothing triggers the next launch early:
+// its waiting blocks would keep other handles' kernels off the SMs (three
+// handles in rotation, 50k bodies: 36.6 -> 51.6 us a step).
+__device__ __forceinline__ void wait_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                           A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Reciprocal square root with subnormal inputs flushed to zero, which drops
 // the subnormal-input handling around each hardware rsqrt.  It changes a
 // result only for |r|^2 + eps^2 below 1.2e-38 (coincident bodies without

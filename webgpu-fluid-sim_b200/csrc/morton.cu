@@ -83,6 +83,7 @@ __device__ __forceinline__ void warp_box(float& a, float& b, float& c, float& d)
 // scratch->bbox = ordered max of {-x, -y, x, y}; zeroed by the step memset.
 __global__ void __launch_bounds__(256) bbox_kernel(const float4* __restrict__ pos2, uint32_t n,
                                                    StepScratch* scratch) {
+    wait_previous_kernel();
     float nx = -INFINITY, ny = -INFINITY, px = -INFINITY, py = -INFINITY;
     const uint32_t pairs = n / 2;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
@@ -115,7 +116,7 @@ void launch_bbox(const DeviceBuffers& b, cudaStream_t s) {
     int blocks = (int)((pairs + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
-    bbox_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const float4*>(b.pos), b.n, b.scratch);
+    launch_chained(bbox_kernel, blocks, 256, 0, s, reinterpret_cast<const float4*>(b.pos), b.n, b.scratch);
 }
 
 // ---- Morton encode + digit histograms --------------------------------------
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(256) encode_kernel(const float4* __restrict__ 
                                                      StepScratch* scratch,
                                                      const float* __restrict__ mass,
                                                      float4* __restrict__ xm) {
+    wait_previous_kernel();
     constexpr int P = (int)sizeof(K);  // digit passes = key bytes
     __shared__ uint32_t sh[P][kRadix];
     for (int i = threadIdx.x; i < P * kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
@@ -214,10 +216,10 @@ void launch_encode(const DeviceBuffers& b, int domain, cudaStream_t s) {
     if (blocks < 1) blocks = 1;
     const float4* p2 = reinterpret_cast<const float4*>(b.pos);
     if (b.key_bytes == 8)
-        encode_kernel<uint64_t><<<blocks, 256, 0, s>>>(p2, b.n, (uint64_t*)b.codes, domain, b.scratch,
+        launch_chained(encode_kernel<uint64_t>, blocks, 256, 0, s, p2, b.n, (uint64_t*)b.codes, domain, b.scratch,
                                                        b.mass, b.xm);
     else
-        encode_kernel<uint32_t><<<blocks, 256, 0, s>>>(p2, b.n, (uint32_t*)b.codes, domain, b.scratch,
+        launch_chained(encode_kernel<uint32_t>, blocks, 256, 0, s, p2, b.n, (uint32_t*)b.codes, domain, b.scratch,
                                                        b.mass, b.xm);
 }
 
@@ -227,6 +229,7 @@ void launch_encode(const DeviceBuffers& b, int domain, cudaStream_t s) {
 __global__ void __launch_bounds__(256) bbox_ensemble_kernel(const float2* __restrict__ pos,
                                                             const uint32_t* __restrict__ body_sys,
                                                             uint32_t n, uint32_t* __restrict__ sys_bbox) {
+    wait_previous_kernel();
     const unsigned FULL = 0xFFFFFFFFu;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
@@ -255,7 +258,7 @@ void launch_bbox_ensemble(const DeviceBuffers& b, cudaStream_t s) {
     if (b.n == 0) return;
     int blocks = (int)((b.n + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
-    bbox_ensemble_kernel<<<blocks, 256, 0, s>>>(b.pos, b.body_sys, b.n, b.sys_bbox);
+    launch_chained(bbox_ensemble_kernel, blocks, 256, 0, s, b.pos, b.body_sys, b.n, b.sys_bbox);
 }
 
 // key = (system << 32) | morton32 over the system's box (same quantisation as
@@ -268,6 +271,7 @@ __global__ void __launch_bounds__(256) encode_ensemble_kernel(const float2* __re
                                                               StepScratch* scratch,
                                                               const float* __restrict__ mass,
                                                               float4* __restrict__ xm) {
+    wait_previous_kernel();
     __shared__ uint32_t sh[8][kRadix];
     for (int i = threadIdx.x; i < 8 * kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
     __syncthreads();
@@ -312,7 +316,7 @@ void launch_encode_ensemble(const DeviceBuffers& b, cudaStream_t s) {
     if (b.n == 0) return;
     int blocks = (int)((b.n + 255) / 256);
     if (blocks > 148 * encode_blocks_per_sm(b.n)) blocks = 148 * encode_blocks_per_sm(b.n);
-    encode_ensemble_kernel<<<blocks, 256, 0, s>>>(b.pos, b.body_sys, b.sys_bbox, b.n, b.sort_passes,
+    launch_chained(encode_ensemble_kernel, blocks, 256, 0, s, b.pos, b.body_sys, b.sys_bbox, b.n, b.sort_passes,
                                                   (uint64_t*)b.codes, b.scratch, b.mass, b.xm);
 }
 
@@ -321,6 +325,7 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(float2* __restrict__ po
                                                          float2* __restrict__ vel,
                                                          const float2* __restrict__ acc, uint32_t n,
                                                          float dt, float hdt) {
+    wait_previous_kernel();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float2 v = vel[i], a = acc[i], p = pos[i];
         v.x = __fadd_rn(v.x, __fmul_rn(a.x, hdt));
@@ -338,6 +343,7 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(float2* __restrict__ po
 static_assert(sizeof(StepScratch) % 4 == 0, "scratch is cleared in 4-byte words");
 __global__ void __launch_bounds__(256) zero_step_kernel(uint32_t* __restrict__ scratch, uint32_t words,
                                                         uint4* __restrict__ status, size_t quads) {
+    wait_previous_kernel();
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = t; i < words; i += stride) scratch[i] = 0u;
@@ -353,7 +359,7 @@ void launch_zero_step(const DeviceBuffers& b, cudaStream_t s) {
     size_t blocks = (work + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
-    zero_step_kernel<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<uint32_t*>(b.scratch), words,
+    launch_chained(zero_step_kernel, (unsigned)blocks, 256, 0, s, reinterpret_cast<uint32_t*>(b.scratch), words,
                                                       reinterpret_cast<uint4*>(b.status), quads);
 }
 
@@ -361,7 +367,7 @@ void launch_kick_drift(const DeviceBuffers& b, float dt, cudaStream_t s) {
     if (b.n == 0) return;
     int blocks = (int)((b.n + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
-    kick_drift_kernel<<<blocks, 256, 0, s>>>(b.pos, b.vel, b.acc, b.n, dt, 0.5f * dt);
+    launch_chained(kick_drift_kernel, blocks, 256, 0, s, b.pos, b.vel, b.acc, b.n, dt, 0.5f * dt);
 }
 
 }  // namespace bh

@@ -68,6 +68,7 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
                 K* __restrict__ keys_out, uint32_t* __restrict__ ids_out, uint32_t n, int pass,
                 StepScratch* __restrict__ scratch, uint32_t* __restrict__ status, uint32_t tiles,
                 uint32_t* __restrict__ err, uint32_t spin_cap, uint32_t debug_flags) {
+    wait_previous_kernel();
     constexpr int W = kSortThreads / 32;
     constexpr int kSortTile = kSortThreads * kSortItems;
     __shared__ uint32_t s_whist[W][kRadix];
@@ -258,12 +259,10 @@ static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
     uint32_t* iout = b.ids_alt;
     for (int p = 0; p < passes; ++p) {
         if (p == 0)
-            onesweep_kernel<K, ITEMS, true><<<b.tiles, kSortThreads, smem, s>>>(
-                kin, nullptr, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
+            launch_chained(onesweep_kernel<K, ITEMS, true>, b.tiles, kSortThreads, smem, s, (const K*)kin, (const uint32_t*)nullptr, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
                 b.debug_flags);
         else
-            onesweep_kernel<K, ITEMS, false><<<b.tiles, kSortThreads, smem, s>>>(
-                kin, iin, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
+            launch_chained(onesweep_kernel<K, ITEMS, false>, b.tiles, kSortThreads, smem, s, (const K*)kin, (const uint32_t*)iin, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
                 b.debug_flags);
         K* tk = kin; kin = kout; kout = tk;
         uint32_t* ti = iin; iin = iout; iout = ti;

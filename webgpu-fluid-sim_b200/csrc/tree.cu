@@ -50,14 +50,14 @@ static void launch_typed(const DeviceBuffers& b, int fp64_levels, cudaStream_t s
     a.err = b.err;
     if (!split_build(b.n, b.debug_flags)) {
         constexpr uint32_t B = build_block<false>();
-        build_fill_kernel<K, false><<<(b.n + B - 1) / B, B, sizeof(BuildShared<K, B>), s>>>(a);
+        launch_chained(build_fill_kernel<K, false>, (b.n + B - 1) / B, B, sizeof(BuildShared<K, B>), s, a);
         return;
     }
     a.frontier = b.frontier;
     a.frontier_count = &b.scratch->frontier_ctr;
     constexpr uint32_t B = build_block<true>();
     const uint32_t grid = (b.n + B - 1) / B;
-    build_fill_kernel<K, true><<<grid, B, sizeof(BuildShared<K, B>), s>>>(a);
+    launch_chained(build_fill_kernel<K, true>, grid, B, sizeof(BuildShared<K, B>), s, a);
     // Frontier nodes number far fewer than bodies (a handful per CTA), but
     // only the device knows how many: a resident grid strides over them.
     static int blocks_per_sm[64] = {};
@@ -72,7 +72,7 @@ static void launch_typed(const DeviceBuffers& b, int fp64_levels, cudaStream_t s
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint32_t blocks = (uint32_t)(sms * bps);
     if (blocks > grid) blocks = grid;
-    build_climb_kernel<K><<<blocks, kClimbBlock, 0, s>>>(a);
+    launch_chained(build_climb_kernel<K>, blocks, kClimbBlock, 0, s, a);
 }
 
 // Reference-layout internal-node arrays from the packed records: node4

@@ -462,6 +462,7 @@ build_fill_kernel(const BuildArgs<K> A) {
     extern __shared__ __align__(16) unsigned char build_smem[];
     BuildShared<K, B>& S = *reinterpret_cast<BuildShared<K, B>*>(build_smem);
 
+    wait_previous_kernel();
     const uint32_t n = A.n;
     if (step_failed(A.err)) return;  // uniform over the block
     const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -590,6 +591,7 @@ build_fill_kernel(const BuildArgs<K> A) {
 template <typename K>
 __global__ void __launch_bounds__(kClimbBlock)
 build_climb_kernel(const BuildArgs<K> A) {
+    wait_previous_kernel();
     if (step_failed(A.err)) return;
     const uint32_t count = *A.frontier_count;
     const uint32_t n = A.n, nm1 = n - 1;

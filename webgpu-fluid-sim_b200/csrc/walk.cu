@@ -92,6 +92,7 @@ walk_kernel(const float4* __restrict__ node4, const uint2* __restrict__ children
     using Mask = typename MaskOf<T>::type;
     __shared__ uint32_t s_node[kExactWarps][kExactStack];
     __shared__ Mask s_mask[kExactWarps][kExactStack];
+    wait_previous_kernel();
     if (step_failed(err)) return;  // the tree of this step was not built
     const int stack_cap = (P.stack_cap > 0 && P.stack_cap < kExactStack) ? P.stack_cap : kExactStack;
     const unsigned FULL = 0xFFFFFFFFu;
@@ -278,7 +279,7 @@ static void launch_tb(const DeviceBuffers& b, const WalkParams& p, cudaStream_t 
     constexpr uint32_t per_block = kExactWarps * T;
     const uint32_t blocks = (b.n + per_block - 1) / per_block;
 #define BH_WALK(PL, BK)                                                                      \
-    walk_kernel<MODE, PL, BK, T, B, COUNT><<<blocks, kExactWarps * 32, 0, s>>>(               \
+    launch_chained(walk_kernel<MODE, PL, BK, T, B, COUNT>, blocks, kExactWarps * 32, 0, s,    \
         b.node4, b.children, b.range, b.ids, b.pos, b.vel, b.acc, p, b.err)
     if (p.plummer) {
         if (buckets) BH_WALK(true, true); else BH_WALK(true, false);

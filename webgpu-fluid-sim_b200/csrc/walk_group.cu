@@ -169,6 +169,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
     constexpr int NP = (BPL + 1) / 2;  // packed pairs per lane
     extern __shared__ __align__(16) unsigned char walk_smem[];
     GroupSmem* smem = reinterpret_cast<GroupSmem*>(walk_smem);
+    wait_previous_kernel();
     if (step_failed(err)) return;  // the tree of this step was not built
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     GroupSmem& S = smem[warp];
@@ -695,7 +696,7 @@ static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, cud
     const uint32_t need = q.split ? b.n : (b.n + warps - 1) / warps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
-    walk_group_kernel<BPL, MP, PL, FAR, COUNT><<<blocks, warps * 32, smem, s>>>(
+    launch_chained(walk_group_kernel<BPL, MP, PL, FAR, COUNT>, blocks, warps * 32, smem, s,
         b.gnode, b.node4, b.groups, b.ids, b.pos, b.vel, b.acc, q, b.err);
 }
 
