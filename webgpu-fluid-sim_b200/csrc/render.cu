@@ -49,13 +49,25 @@ struct RenderParams {
 constexpr int kSplatThreads = 256;
 constexpr int kToneThreads = 256;
 
-// density.wgsl:39-97, one warp per 32 bodies.  Each lane sets up its own
-// body once (centre and radius in pixels, pixel bounds, weight) and the warp
-// then splats the 32 bodies one after the other, the setup of each shuffled
-// from its lane.  The lanes cover the body's pixel rectangle in 8 x 4 tiles,
-// with integer pixel indices and exactly representable float pixel centres
-// stepped by additions: no division or conversion per pixel, one hardware
-// exponential per covered pixel.
+// density.wgsl:39-97.  Each lane sets up its own body once (centre and radius
+// in pixels, pixel bounds, weight); the setups are shuffled to the lanes that
+// splat.  Small discs (at most kSmallSpan pixels wide and high: all but a
+// scene's few large bodies) go four at a time, eight lanes each, a pixel
+// column per lane, row by row, so a row's adds reach the L2 as one or two
+// 32-byte requests.  Large discs go one after the other, the whole warp in
+// 8 x 4 tiles.  Pixel centres are exactly representable floats and every
+// pixel's weight is computed the same way on both paths: no division or
+// conversion, one hardware exponential.
+// (The warp on one disc at a time spent 78 warp instructions on a 5 x 5 pixel
+// disc, mostly idle lanes and shuffles, and was bound by their issue.  Now the
+// L2's requests bound it: a frame of 800k bodies at 1920 x 1080, with the tone
+// table below, 91 -> 48 us; zoomed out until all of them share a few thousand
+// pixels, where the adds meet each other, 109-138 us before and 112 now.  A
+// disc per lane with one 16-byte vector reduction per four pixels needs as
+// many requests and meets itself more often: 48 and 135 us; scalar reductions
+// 89 and 249 us.  16 / 4 / 2 blocks per SM: 46 / 50 / 60 and 110 / 137 / 139.)
+constexpr int kSmallSpan = 8;
+constexpr uint32_t kSplatBlocksPerSm = 8;
 __global__ void __launch_bounds__(kSplatThreads)
 splat_kernel(const float2* __restrict__ pos, const float* __restrict__ radius_mul, uint32_t n,
              const RenderParams P, float* __restrict__ density) {
@@ -97,28 +109,50 @@ splat_kernel(const float2* __restrict__ pos, const float* __restrict__ radius_mu
             inv_r = __frcp_rn(R);
             bw = __fmul_rn(rm > 1.0f ? 0.1f : 0.02f, zoom_scale);  // density.wgsl:90-95
         }
-        const int cnt = (n - base) < 32u ? (int)(n - base) : 32;
-        for (int k = 0; k < cnt; ++k) {
+        // uv and r^2 = |uv|^2; discard outside the disc (density.wgsl:73-78);
+        // w = exp(-k r^2), k = 10 (density.wgsl:81-82): the hardware exponential,
+        // relative error ~1e-6 over r^2 in [0, 1]
+        auto splat = [](float* px, float ux2, float uy2, float w) {
+            const float r2 = __fadd_rn(ux2, uy2);
+            if (!(r2 > 1.0f)) atomicAdd(px, __fmul_rn(w, __expf(__fmul_rn(-10.0f, r2))));
+        };
+        auto square = [](float c, float centre, float ir) {
+            const float u = __fmul_rn(__fsub_rn(c, centre), ir);
+            return __fmul_rn(u, u);
+        };
+        const bool drawn = ia <= ib;
+        const bool small = drawn && ib - ia < kSmallSpan && jb - ja < kSmallSpan;
+        const unsigned smalls = __ballot_sync(FULL, small);
+        const int gx = lane & 7, gy = lane >> 3;
+#pragma unroll 1
+        for (int it = 0; it < 8; ++it) {
+            const int k = 4 * it + gy;
             const int kia = __shfl_sync(FULL, ia, k), kib = __shfl_sync(FULL, ib, k);
             const int kja = __shfl_sync(FULL, ja, k), kjb = __shfl_sync(FULL, jb, k);
-            if (kia > kib) continue;  // nothing on screen (uniform)
+            const float kcx = __shfl_sync(FULL, cpx, k), kcy = __shfl_sync(FULL, cpy, k);
+            const float kir = __shfl_sync(FULL, inv_r, k), kbw = __shfl_sync(FULL, bw, k);
+            const int i = kia + gx;
+            if (((smalls >> k) & 1u) && i <= kib) {
+                const float ux2 = square((float)i + 0.5f, kcx, kir);
+                float yc = (float)kja + 0.5f;
+                float* px = density + (size_t)kja * P.w + i;
+                for (int j = kja; j <= kjb; ++j, yc = __fadd_rn(yc, 1.0f), px += P.w)
+                    splat(px, ux2, square(yc, kcy, kir), kbw);
+            }
+        }
+        for (unsigned large = __ballot_sync(FULL, drawn && !small); large; large &= large - 1u) {
+            const int k = __ffs(large) - 1;
+            const int kia = __shfl_sync(FULL, ia, k), kib = __shfl_sync(FULL, ib, k);
+            const int kja = __shfl_sync(FULL, ja, k), kjb = __shfl_sync(FULL, jb, k);
             const float kcx = __shfl_sync(FULL, cpx, k), kcy = __shfl_sync(FULL, cpy, k);
             const float kir = __shfl_sync(FULL, inv_r, k), kbw = __shfl_sync(FULL, bw, k);
             float yc = (float)(kja + ty) + 0.5f;
             for (int j = kja + ty; j <= kjb; j += 4, yc = __fadd_rn(yc, 4.0f)) {
-                // uv and r^2 = |uv|^2; discard outside the disc (density.wgsl:73-78)
-                const float uy = __fmul_rn(__fsub_rn(yc, kcy), kir);
-                const float uy2 = __fmul_rn(uy, uy);
+                const float uy2 = square(yc, kcy, kir);
                 float* row = density + (size_t)j * P.w;
                 float xc = (float)(kia + tx) + 0.5f;
-                for (int i = kia + tx; i <= kib; i += 8, xc = __fadd_rn(xc, 8.0f)) {
-                    const float ux = __fmul_rn(__fsub_rn(xc, kcx), kir);
-                    const float r2 = __fadd_rn(__fmul_rn(ux, ux), uy2);
-                    if (r2 > 1.0f) continue;
-                    // w = exp(-k r^2), k = 10 (density.wgsl:81-82): the hardware
-                    // exponential, relative error ~1e-6 over r^2 in [0, 1]
-                    atomicAdd(&row[i], __fmul_rn(kbw, __expf(__fmul_rn(-10.0f, r2))));
-                }
+                for (int i = kia + tx; i <= kib; i += 8, xc = __fadd_rn(xc, 8.0f))
+                    splat(&row[i], square(xc, kcx, kir), uy2, kbw);
             }
         }
     }
@@ -146,17 +180,41 @@ __device__ __forceinline__ unsigned char unorm8(float c) {
     return (unsigned char)__float2uint_rn(__fmul_rn(fminf(fmaxf(c, 0.0f), 1.0f), 255.0f));
 }
 
-// tone_map.wgsl:63-84, one thread per pixel.
-__global__ void __launch_bounds__(kToneThreads)
-tone_map_kernel(const float* __restrict__ density, uint32_t pixels, uchar4* __restrict__ image) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= pixels) return;
-    const float d = __half2float(__float2half_rn(__ldg(&density[p])));  // r16float texel
+// tone_map.wgsl:63-84 of one r16float texel.
+__device__ __forceinline__ uchar4 tone_map(__half texel) {
+    const float d = __half2float(texel);
     const float x = __fmul_rn(8.0f, d);                                  // exposure 8
     const float mapped = __fdiv_rn(x, __fadd_rn(1.0f, x));               // Reinhard
     const float g = powf(fminf(fmaxf(mapped, 0.0f), 1.0f), (float)(1.0 / 2.2));
     const float3 c = colormap(g);
-    image[p] = make_uchar4(unorm8(c.x), unorm8(c.y), unorm8(c.z), 255);
+    return make_uchar4(unorm8(c.x), unorm8(c.y), unorm8(c.z), 255);
+}
+
+// The tone curve has one value per r16float texel: all 65,536 of them, computed
+// once when a renderer is made, serve every frame (256 KB, in the L2).  Two
+// hundred instructions a pixel -- two divisions and a power -- become a load:
+// tone map 18 -> 7 us of a 1920 x 1080 frame.
+constexpr uint32_t kToneEntries = 1u << 16;
+__global__ void __launch_bounds__(kToneThreads) tone_table_kernel(uchar4* __restrict__ table) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < kToneEntries) table[t] = tone_map(__ushort_as_half((unsigned short)t));
+}
+
+// One thread per four pixels.
+__global__ void __launch_bounds__(kToneThreads)
+tone_map_kernel(const float* __restrict__ density, uint32_t pixels,
+                const uchar4* __restrict__ table, uchar4* __restrict__ image) {
+    auto texel = [&](float d) {
+        return __ldg(reinterpret_cast<const uint32_t*>(table) +
+                     __half_as_ushort(__float2half_rn(d)));
+    };
+    const uint32_t p = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (p + 3u < pixels) {
+        const float4 d = *reinterpret_cast<const float4*>(density + p);
+        *reinterpret_cast<uint4*>(image + p) = make_uint4(texel(d.x), texel(d.y), texel(d.z), texel(d.w));
+    } else {
+        for (uint32_t q = p; q < pixels; ++q) reinterpret_cast<uint32_t*>(image)[q] = texel(density[q]);
+    }
 }
 
 }  // namespace bh
@@ -172,6 +230,7 @@ struct bh_renderer {
     double cam[4] = {0.0, 0.0, 10.0, 10.0};
     float* density = nullptr;
     uint8_t* image = nullptr;
+    uchar4* tone = nullptr;  // the tone curve by r16float texel
     std::string err;
 };
 
@@ -198,14 +257,15 @@ static int alloc_targets(bh_renderer* r, uint32_t w, uint32_t h) {
     r->density = nullptr;
     r->image = nullptr;
     const size_t px = (size_t)w * h;
+    const size_t quads = (px + 3) & ~(size_t)3;  // both targets start and end on 16 bytes
     void* mem = nullptr;
-    e = cudaMalloc(&mem, px * sizeof(float) + px * 4);
+    e = cudaMalloc(&mem, quads * sizeof(float) + quads * 4);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rcuda(r, e, "cudaMalloc(render targets)");
     }
     r->density = static_cast<float*>(mem);
-    r->image = reinterpret_cast<uint8_t*>(r->density + px);
+    r->image = reinterpret_cast<uint8_t*>(r->density + quads);
     r->width = w;
     r->height = h;
     // resizeCanvasToDisplaySize (renderer.ts:242-246): keep the vertical half
@@ -221,8 +281,23 @@ extern "C" int bh_renderer_create(bh_sim* sim, uint32_t width, uint32_t height, 
     bh_renderer* r = new bh_renderer();
     r->sim = sim;
     r->device = v.device;
-    const int st = alloc_targets(r, width, height);
+    int st = alloc_targets(r, width, height);
+    if (st == BH_OK) {
+        cudaError_t e = cudaMalloc((void**)&r->tone, bh::kToneEntries * sizeof(uchar4));
+        if (e == cudaSuccess) {
+            // on the simulation's stream, before any frame
+            bh::tone_table_kernel<<<bh::kToneEntries / bh::kToneThreads, bh::kToneThreads, 0,
+                                    v.stream>>>(r->tone);
+            e = cudaGetLastError();
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            st = rcuda(r, e, "tone table");
+        }
+    }
     if (st != BH_OK) {
+        cudaFree(r->density);
+        cudaFree(r->tone);
         delete r;
         return st;
     }
@@ -232,9 +307,10 @@ extern "C" int bh_renderer_create(bh_sim* sim, uint32_t width, uint32_t height, 
 
 extern "C" int bh_renderer_destroy(bh_renderer* r) {
     if (!r) return BH_OK;
-    if (r->density) {
+    if (r->density || r->tone) {
         cudaSetDevice(r->device);
         cudaFree(r->density);
+        cudaFree(r->tone);
     }
     delete r;
     return BH_OK;
@@ -304,14 +380,15 @@ extern "C" int bh_renderer_frame(bh_renderer* r) {
     if (v.n > 0) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
-        uint32_t blocks = (uint32_t)sms * 8u;
+        uint32_t blocks = (uint32_t)sms * bh::kSplatBlocksPerSm;
         const uint32_t need = (v.n + bh::kSplatThreads - 1) / bh::kSplatThreads;
         if (blocks > need) blocks = need;
         bh::splat_kernel<<<blocks, bh::kSplatThreads, 0, v.stream>>>(v.pos, v.radius, v.n, P,
                                                                      r->density);
     }
-    bh::tone_map_kernel<<<(uint32_t)((px + bh::kToneThreads - 1) / bh::kToneThreads),
-                          bh::kToneThreads, 0, v.stream>>>(r->density, (uint32_t)px,
+    const size_t quads = (px + 3) / 4;
+    bh::tone_map_kernel<<<(uint32_t)((quads + bh::kToneThreads - 1) / bh::kToneThreads),
+                          bh::kToneThreads, 0, v.stream>>>(r->density, (uint32_t)px, r->tone,
                                                            reinterpret_cast<uchar4*>(r->image));
     e = cudaGetLastError();
     if (e != cudaSuccess) return rcuda(r, e, "render kernels launch");
