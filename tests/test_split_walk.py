@@ -1,5 +1,6 @@
 """Few groups: a block's warps share one group's lists (fewer than 8 groups per
-SM; a group holds about 0.7 of its 32 x bodiesPerLane bodies).  Body counts on
+SM, and two warps below 16 where the caller waits for the forces; a group
+holds about 0.7 of its 32 x bodiesPerLane bodies).  Body counts on
 both sides of the rule and every block shape against the oracle's walk of the
 same groups: the interactions are the same, FP32 terms within 1e-6, so sums
 within 1e-5 of the larger of the body's and the median acceleration for all
@@ -19,12 +20,12 @@ def _edge(bpl, per_sm):
     return int(0.7 * 32 * bpl * per_sm * torch.cuda.get_device_properties(0).multi_processor_count)
 
 
-@pytest.mark.parametrize("bpl", [1, 2])
+@pytest.mark.parametrize("bpl,per_sm", [(1, 8), (2, 8), (1, 16)])
 @pytest.mark.parametrize("off", [-1, 1])
 @pytest.mark.parametrize("far", [0.0, 0.4])
-def test_walk_on_both_sides_of_the_rule(bh, orc, bpl, off, far):
+def test_walk_on_both_sides_of_the_rule(bh, orc, bpl, per_sm, off, far):
     sim = bh.Simulation(bh.Config(**CFG, bodiesPerLane=bpl, farAlpha=far))
-    sim.setNumBodies(_edge(bpl, 8) + off)
+    sim.setNumBodies(_edge(bpl, per_sm) + off)
     sim.setScenario("uniform-disk-kepler", 3)
     mass, pos, vel = sim.download()
     acc = sim.computeAccelerations().astype(np.float64)

@@ -178,7 +178,8 @@ struct WalkParams {
     int multipole;    // 1 or 2
     int bpl;          // bodies per lane
     unsigned int* group_ctr;  // dynamic group counter (zeroed per step)
-    int split = 0;    // 1 = a block's warps share one group (set by the launcher)
+    int latency = 0;  // the caller waits for this walk alone (see split_groups)
+    int split = 0;    // VJP: 1 = a block's warps share one group (set by the launcher)
     // ensemble: a group only sees its own system's slot range
     uint32_t num_systems;
     const uint32_t* sys_off;

@@ -41,11 +41,15 @@ struct bh_sim {
     void* arena = nullptr;
     size_t arena_bytes = 0;
     bool acc_valid = false;
+    // The call in progress waits for its result (forces, gradients): walks may
+    // spend more work to be done sooner.
+    bool waited_for = false;
     // graphs: [0] plain, [1] with event-record nodes at the stage boundaries;
     // for the first step after an upload still being copied (see bh_upload):
     // [2] the tree stages, [3] the walk, [4] the tree stages up to the sort
-    // without packed leaf records, [5] the build reading masses and positions
-    static constexpr int kGraphs = 6;
+    // without packed leaf records, [5] the build reading masses and positions;
+    // [6] plain, for calls that wait
+    static constexpr int kGraphs = 7;
     cudaGraph_t graph[kGraphs] = {};
     cudaGraphExec_t exec[kGraphs] = {};
     // Uploads are staged: bh_upload copies each array into its staging
@@ -102,6 +106,13 @@ struct bh_sim {
 };
 
 static thread_local std::string g_err;
+
+// Marks a call that waits for its result, for the scope it enqueues work in.
+struct Waiting {
+    bh_sim* s;
+    explicit Waiting(bh_sim* sim) : s(sim) { s->waited_for = true; }
+    ~Waiting() { s->waited_for = false; }
+};
 
 // Order the handle's stream after uploads still in flight on the copy
 // stream.  Every entry point calls settle_uploads (through BH_HANDLE) before
@@ -473,6 +484,7 @@ static bh::WalkParams walk_params(const bh_sim* s, int mode) {
     p.slot_lo = integrating ? s->shard_lo : 0u;
     p.slot_hi = integrating ? s->shard_hi : 0xFFFFFFFFu;
     p.stack_cap = (int)s->debug_stack_cap;
+    p.latency = s->waited_for;
     p.far_alpha2 = c.walk_mode == BH_WALK_GROUP ? c.far_alpha * c.far_alpha : 0.0f;
     return p;
 }
@@ -1019,7 +1031,7 @@ static int step_once(bh_sim* s) {
         return BH_OK;
     }
     if (s->cfg.use_graphs) {
-        const int v = ev ? 1 : 0;
+        const int v = ev ? 1 : (s->waited_for ? 6 : 0);
         if (!s->exec[v]) {
             int rc = capture_graph(s, v);
             if (rc != BH_OK) return rc;
@@ -1091,13 +1103,15 @@ extern "C" int bh_sync(bh_sim* s) {
 extern "C" int bh_compute_accelerations(bh_sim* s, float* acc_host) {
     BH_HANDLE(s);
     if (s->b.n == 0) return BH_OK;
-    enqueue_forces(s, [](int) {});
+    {
+        Waiting w(s);
+        enqueue_forces(s, [](int) {});
+    }
     BH_CUDA(s, cudaGetLastError());
     if (acc_host)
         BH_CUDA(s, cudaMemcpyAsync(acc_host, s->b.acc, 8 * (size_t)s->b.n, cudaMemcpyDeviceToHost, s->stream));
-    BH_CUDA(s, cudaStreamSynchronize(s->stream));
     s->acc_valid = true;
-    return check_device_errors(s);
+    return check_device_errors(s);  // synchronises once, for the copy and the error word
 }
 
 // ---- adjoint (extension) -----------------------------------------------------------
@@ -1225,8 +1239,7 @@ extern "C" int bh_force_vjp(bh_sim* s, const float* abar, float* xbar, float* mb
     BH_CUDA(s, cudaGetLastError());
     if (xbar) BH_CUDA(s, cudaMemcpyAsync(xbar, a.xbar, 8 * (size_t)n, cudaMemcpyDeviceToHost, s->stream));
     if (mbar) BH_CUDA(s, cudaMemcpyAsync(mbar, a.mbar, 4 * (size_t)n, cudaMemcpyDeviceToHost, s->stream));
-    BH_CUDA(s, cudaStreamSynchronize(s->stream));
-    return check_device_errors(s);
+    return check_device_errors(s);  // synchronises
 }
 
 extern "C" int bh_rollout_grad(bh_sim* s, uint32_t steps, uint32_t checkpoint_every,
@@ -1247,6 +1260,7 @@ extern "C" int bh_rollout_grad(bh_sim* s, uint32_t steps, uint32_t checkpoint_ev
     bh_sim::Adjoint& a = s->adj;
     cudaStream_t st = s->stream;
     const size_t vb = 8 * (size_t)n;
+    Waiting waiting(s);  // every step of the rollout and its replays walks alike
     const float dt = s->cfg.delta_time, h = 0.5f * dt;
     BH_CUDA(s, cudaMemcpyAsync(a.target, target_pos, vb, cudaMemcpyHostToDevice, st));
     // Forward: T steps, saving (x, v) at every checkpoint.  The last segment
@@ -1312,9 +1326,9 @@ extern "C" int bh_rollout_grad(bh_sim* s, uint32_t steps, uint32_t checkpoint_ev
     BH_CUDA(s, cudaMemcpyAsync(s->b.pos, a.fin_pos, vb, cudaMemcpyDeviceToDevice, st));
     BH_CUDA(s, cudaMemcpyAsync(s->b.vel, a.fin_vel, vb, cudaMemcpyDeviceToDevice, st));
     s->acc_valid = false;
-    BH_CUDA(s, cudaStreamSynchronize(st));
+    rc = check_device_errors(s);  // synchronises
     if (loss) *loss = (float)L;
-    return check_device_errors(s);
+    return rc;
 }
 
 extern "C" int bh_walk_stats(bh_sim* s, uint64_t* node_visits, uint64_t* multipole_interactions,

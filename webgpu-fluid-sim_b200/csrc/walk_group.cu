@@ -160,7 +160,7 @@ constexpr int walk_min_blocks(int bpl) { return bpl >= 4 ? BH_WALK_MIN_BLOCKS_12
 // cost 5% at 800k and 16.8M bodies, 8% for 64-body groups).  Shared memory:
 // one GroupSmem per warp, dynamic (the block shape is chosen at
 // launch).
-template <int BPL, int MP, bool PLUMMER, bool FAR, bool COUNT>
+template <int BPL, int MP, bool PLUMMER, bool FAR, bool COUNT, bool SPLIT>
 __global__ void __launch_bounds__(walk_max_threads(BPL), walk_min_blocks(BPL))
 walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ node4,
                   const uint2* __restrict__ groups, const uint32_t* __restrict__ ids,
@@ -176,11 +176,10 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t n = P.n, nm1 = n - 1;
-    // Split walk (few groups): the block's warps walk one group together.  Each
+    // SPLIT (few groups): the block's warps walk one group together.  Each
     // does the whole traversal, and evaluates every turn_mask+1-th batch.
-    const bool split = !COUNT && P.split;
-    const int turn_mask = split ? (int)(blockDim.x >> 5) - 1 : 0;
-    const int my_turn = split ? warp : 0;
+    const int turn_mask = SPLIT ? (int)(blockDim.x >> 5) - 1 : 0;
+    const int my_turn = SPLIT ? warp : 0;
     const uint32_t ngroups = P.group_ctr[1];  // written by the build kernel
     const float th2 = __fmul_rn(P.theta, P.theta);
     const float eps2 = P.eps2, ecoef = P.eps_coef;
@@ -192,7 +191,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
 
     while (true) {
         uint32_t g = 0;
-        if (split) {
+        if (SPLIT) {
             __syncthreads();  // the previous group's sums have been read
             if (threadIdx.x == 0) S.slot[0] = atomicAdd(P.group_ctr, 1u);
             __syncthreads();
@@ -472,7 +471,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             while (nn >= 32 || (last && nn > 0)) {
                 const int cnt = nn < 32 ? nn : 32;
                 nn -= cnt;
-                if ((turn++ & turn_mask) != my_turn) continue;
+                if (SPLIT && (turn++ & turn_mask) != my_turn) continue;
                 float4 mom = make_float4(kFarAway, kFarAway, 0.f, 0.f), tail = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < cnt) ldg_half(&gnode[S.near[nn + lane]].mom, mom, tail);
                 // {com, mass, Sxx}, {Sxy, Syy}: -Q' = tr(S) I - 3S
@@ -503,7 +502,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 // the bodies of up to 32 ranges: one exclusive scan of their counts
                 const int cnt = nr < 32 ? nr : 32;
                 nr -= cnt;
-                if ((turn++ & turn_mask) != my_turn) continue;
+                if (SPLIT && (turn++ & turn_mask) != my_turn) continue;
                 const uint32_t first = lane < cnt ? S.first[nr + lane] : 0u;
                 const uint32_t c = lane < cnt ? S.count[nr + lane] : 0u;
                 uint32_t incl = c;
@@ -521,7 +520,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 while (nf >= 64 || (last && nf > 0)) {
                     const int cnt = nf < 64 ? nf : 64;
                     nf -= cnt;
-                    if ((turn++ & turn_mask) != my_turn) continue;
+                    if (SPLIT && (turn++ & turn_mask) != my_turn) continue;
                     far_batch(gnode, S.far + nf, cacc, lane, cnt, gcx, gcy, far_rg2, eps2);
                     if (counting) c_far += (unsigned long long)cnt;
                     far_used = true;
@@ -596,7 +595,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             ax[k] = far_used ? __fadd_rn(ax[k], fx[k]) : ax[k];
             ay[k] = far_used ? __fadd_rn(ay[k], fy[k]) : ay[k];
         }
-        if (split) {
+        if (SPLIT) {
             // the warps' shares, added in warp order by the first one
             float2* const mine = reinterpret_cast<float2*>(&S.nodes);
 #pragma unroll
@@ -654,10 +653,13 @@ static int shape_index(int warps) { return warps == 2 ? 0 : (warps == 8 ? 2 : 1)
 template <int BPL, int MP, bool PL, bool FAR>
 static cudaError_t set_walk_attributes() {
     const int smem = (int)(walk_max_threads(BPL) / 32 * sizeof(GroupSmem));
-    cudaError_t e = cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, false>,
+    cudaError_t e = cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, false, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, true>,
+    e = cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, false, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(walk_group_kernel<BPL, MP, PL, FAR, true, false>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
@@ -671,40 +673,47 @@ int walk_group_max_block(int bpl) { return walk_max_threads(bpl >= 4 ? 4 : 2); }
 // 32k 40.3 / 32.9, 65k (10 groups per SM) 52.3 / 55.3; 128-body groups without
 // the far field, 50k 157 / 77, 100k (8 per SM) 199 / 121, 200k 221 / 208; with
 // it 50k 104 / 60, 100k 114 / 98, 200k 121 / 160.
+// From there to 16 groups per SM two warps share one, but only where the caller
+// waits for the result (p.latency): 65k leapfrog 53 -> 47 us, forces of 120k
+// bodies 205 -> 130, 200k 221 -> 180, a 65k rollout's gradient 8.29 -> 7.57 ms;
+// with other work on the GPU the second traversal costs more than it saves
+// (65k steps of three handles in rotation 42 -> 47 us each).
 bool split_groups(uint32_t n, uint32_t gmax, int sms, int per_sm) {
     return (double)n < 0.7 * gmax * per_sm * sms;
 }
 
-template <int BPL, int MP, bool PL, bool FAR, bool COUNT>
-static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, cudaStream_t s) {
+template <int BPL, int MP, bool PL, bool FAR, bool COUNT, bool SPLIT>
+static void launch_c(const DeviceBuffers& b, const WalkParams& p, int warps, int dev, int sms,
+                     cudaStream_t s) {
     static int blocks_per_sm[64][3] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
     const size_t smem = (size_t)warps * sizeof(GroupSmem);
     int& bps = blocks_per_sm[dev & 63][shape_index(warps)];
     if (bps == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &bps, walk_group_kernel<BPL, MP, PL, FAR, COUNT>, warps * 32, smem);
+            &bps, walk_group_kernel<BPL, MP, PL, FAR, COUNT, SPLIT>, warps * 32, smem);
         if (bps < 1) bps = 1;
     }
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // Persistent grid; the number of groups (<= n) is only known on the device.
     uint32_t blocks = (uint32_t)(sms * bps);
-    WalkParams q = p;
-    q.split = !COUNT && split_groups(b.n, 32u * BPL, sms, 8);
-    const uint32_t need = q.split ? b.n : (b.n + warps - 1) / warps;
+    const uint32_t need = SPLIT ? b.n : (b.n + warps - 1) / warps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
-    launch_chained(walk_group_kernel<BPL, MP, PL, FAR, COUNT>, blocks, warps * 32, smem, s,
-        b.gnode, b.node4, b.groups, b.ids, b.pos, b.vel, b.acc, q, b.err);
+    launch_chained(walk_group_kernel<BPL, MP, PL, FAR, COUNT, SPLIT>, blocks, warps * 32, smem, s,
+                   b.gnode, b.node4, b.groups, b.ids, b.pos, b.vel, b.acc, p, b.err);
 }
 
 // The counting walk only when bh_walk_stats asks for it (p.count).
 template <int BPL, int MP, bool PL, bool FAR = false>
 static void launch_t(const DeviceBuffers& b, const WalkParams& p, int warps, cudaStream_t s) {
-    if (p.count) launch_c<BPL, MP, PL, FAR, true>(b, p, warps, s);
-    else launch_c<BPL, MP, PL, FAR, false>(b, p, warps, s);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (p.count) launch_c<BPL, MP, PL, FAR, true, false>(b, p, warps, dev, sms, s);
+    else if (split_groups(b.n, 32u * BPL, sms, 8))
+        launch_c<BPL, MP, PL, FAR, false, true>(b, p, warps, dev, sms, s);
+    else if (p.latency && split_groups(b.n, 32u * BPL, sms, 16))
+        launch_c<BPL, MP, PL, FAR, false, true>(b, p, 2, dev, sms, s);
+    else launch_c<BPL, MP, PL, FAR, false, false>(b, p, warps, dev, sms, s);
 }
 
 template <int BPL>
