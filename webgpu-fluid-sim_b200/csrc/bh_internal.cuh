@@ -240,7 +240,7 @@ struct DeviceBuffers {
     uint32_t* err = nullptr;     // device error word
     uint32_t spin_cap = kSpinCapDefault;  // sort look-back wait bound (spins)
     uint32_t debug_flags = 0;    // kDebug* test hooks
-    int sort_passes = 0;         // 0: one per key byte; ensembles sort fewer (even count)
+    int sort_passes = 0;         // 0: one per key byte; ensembles sort fewer
     // ensemble of independent systems (num_systems = 0: one system)
     uint32_t num_systems = 0;
     const uint32_t* sys_off = nullptr;  // E+1 body offsets (original order = sorted order by system)
@@ -282,6 +282,9 @@ int walk_group_max_block(int bpl);
 cudaError_t build_init_attributes();
 int sort_passes(const DeviceBuffers& b);
 uint32_t sort_tiles(uint32_t n);  // tiles of the sort of n keys
+// Where the encode leaves the keys: an odd number of passes starts in the
+// alternate buffer, so the sorted keys always end in `codes`.
+inline void* sort_input(const DeviceBuffers& b) { return sort_passes(b) & 1 ? b.codes_alt : b.codes; }
 // tree.cu
 void launch_build_fill(const DeviceBuffers& b, int fp64_levels, cudaStream_t s);
 // Bodies from which the build runs as two kernels (local phase + frontier climb).

@@ -436,12 +436,10 @@ static int alloc_buffers(bh_sim* s, uint32_t n) {
         b.sys_off = (uint32_t*)(a + o_soff);
         b.body_sys = (uint32_t*)(a + o_bsys);
         b.sys_bbox = (uint32_t*)(a + o_sbox);
-        // key bits = 32 + bits of the largest system id; an even pass count
-        // lands the sorted keys back in `codes`
+        // key bits = 32 + bits of the largest system id
         int sb = 0;
         while (sb < 32 && ((E - 1) >> sb)) ++sb;
-        int passes = (32 + sb + 7) / 8;
-        b.sort_passes = passes + (passes & 1);
+        b.sort_passes = (32 + sb + 7) / 8;
         // On the handle's stream, after the arena memset above: the stream is
         // non-blocking, so a copy on the legacy stream would not be ordered
         // against that memset (which could then clear the offsets).

@@ -317,7 +317,7 @@ void launch_encode_ensemble(const DeviceBuffers& b, cudaStream_t s) {
     int blocks = (int)((b.n + 255) / 256);
     if (blocks > 148 * encode_blocks_per_sm(b.n)) blocks = 148 * encode_blocks_per_sm(b.n);
     launch_chained(encode_ensemble_kernel, blocks, 256, 0, s, b.pos, b.body_sys, b.sys_bbox, b.n, b.sort_passes,
-                                                  (uint64_t*)b.codes, b.scratch, b.mass, b.xm);
+                                                  (uint64_t*)sort_input(b), b.scratch, b.mass, b.xm);
 }
 
 // ---- leapfrog opening kick + drift (original order, coalesced) -----------

@@ -21,8 +21,8 @@
 //    contiguous per digit.
 //  - Pass 0 does not read ids: it writes the identity permutation of
 //    lbvh.wgsl:68 directly.
-//  - With an even number of passes (4 for 32-bit keys, 8 for 64-bit keys)
-//    the result lands back in the public codes / ids buffers.
+//  - The passes alternate between two buffers and end in the public codes /
+//    ids (an odd number of passes, ensembles only, starts in the others).
 #include <cuda/atomic>
 
 #include "bh_internal.cuh"
@@ -230,7 +230,7 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
     }
 }
 
-// One pass per key byte, or fewer (an even count) when the high bytes are
+// One pass per key byte, or fewer when the high bytes are
 // known to be zero (ensemble keys: system id above a 32-bit Morton code).
 int sort_passes(const DeviceBuffers& b) { return b.sort_passes > 0 ? b.sort_passes : b.key_bytes; }
 
@@ -253,10 +253,11 @@ template <typename K, int ITEMS>
 static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
     const size_t smem = (size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t));
     const int passes = sort_passes(b);
-    K* kin = (K*)b.codes;
-    K* kout = (K*)b.codes_alt;
-    uint32_t* iin = b.ids;
-    uint32_t* iout = b.ids_alt;
+    const bool odd = passes & 1;  // the last pass writes codes / ids
+    K* kin = (K*)sort_input(b);
+    K* kout = (K*)(odd ? b.codes : b.codes_alt);
+    uint32_t* iin = odd ? b.ids_alt : b.ids;
+    uint32_t* iout = odd ? b.ids : b.ids_alt;
     for (int p = 0; p < passes; ++p) {
         if (p == 0)
             launch_chained(onesweep_kernel<K, ITEMS, true>, b.tiles, kSortThreads, smem, s, (const K*)kin, (const uint32_t*)nullptr, kout, iout, b.n, p, b.scratch, b.status, b.tiles, b.err, b.spin_cap,
