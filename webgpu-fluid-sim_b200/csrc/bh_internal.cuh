@@ -180,9 +180,10 @@ struct WalkParams {
     unsigned int* group_ctr;  // dynamic group counter (zeroed per step)
     int latency = 0;  // the caller waits for this walk alone (see split_groups)
     int split = 0;    // VJP: 1 = a block's warps share one group (set by the launcher)
-    // ensemble: a group only sees its own system's slot range
+    // ensemble: a group only sees its own system's subtree
     uint32_t num_systems;
     const uint32_t* sys_off;
+    const uint64_t* sys_keys;  // sorted keys: system id above the Morton code
     // sharding: only groups whose first sorted slot lies in [slot_lo, slot_hi)
     uint32_t slot_lo;
     uint32_t slot_hi;

@@ -476,6 +476,7 @@ static bh::WalkParams walk_params(const bh_sim* s, int mode) {
     p.group_ctr = s->b.scratch ? s->b.scratch->group_ctr : nullptr;
     p.num_systems = s->b.num_systems;
     p.sys_off = s->b.sys_off;
+    p.sys_keys = (const uint64_t*)s->b.codes;
     // Sharding restricts the integrating walk of a step; force evaluations
     // (the first leapfrog force, bh_compute_accelerations) cover every body.
     const bool integrating = mode == bh::kWalkEulerKickDrift || mode == bh::kWalkKdkClose;

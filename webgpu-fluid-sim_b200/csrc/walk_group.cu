@@ -68,8 +68,8 @@
 // warp instructions at 62% of the issue slots, 24 warps per SM, FMA pipe 47%;
 // the last 14% of the launch is the drain of the last groups.  Walk stage
 // before the branch-free step, id lists, packed far batches and passes over
-// one loop -> now: 800k 389 -> 305 us, 16.8M 7.61 -> 5.80 ms, 64-body groups
-// (ensemble of 64 systems, 1.2M bodies) 584 -> 438 us.
+// one loop -> now: 800k 389 -> 296 us, 16.8M 7.61 -> 5.59 ms, 64-body groups
+// (ensemble of 64 systems, 1.2M bodies) 584 -> 388 us.
 #include "bh_internal.cuh"
 #include "far_field.cuh"
 #include "packed.cuh"
@@ -208,18 +208,18 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
         if (grp.x < P.slot_lo || grp.x >= P.slot_hi) continue;  // another shard's group (uniform)
         const uint32_t base = grp.x, nvalid = grp.y;
         const int kmax = (int)((nvalid + 31u) / 32u);  // sub-slots in use (uniform)
-        // Ensemble: the slot range of this group's system (systems stay
-        // contiguous in sorted order because the system id tops every key).
-        uint32_t sys_lo = 0, sys_hi = n;
+        // Ensemble: start at the root of the group's own system.  The system id
+        // tops every key, so a system is one subtree, whose Karras index is its
+        // first or its last slot.  (Started at the common root, with every node
+        // tested against the system's slot range: 435 us, now 388, 64 systems of
+        // 1.2M bodies.)
+        uint32_t root = 0;
         if (P.num_systems > 0) {
-            uint32_t lo = 0, hi = P.num_systems;  // sys_off[lo] <= base < sys_off[hi]
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (__ldg(&P.sys_off[mid]) <= base) lo = mid;
-                else hi = mid;
-            }
-            sys_lo = __ldg(&P.sys_off[lo]);
-            sys_hi = __ldg(&P.sys_off[lo + 1]);
+            const uint32_t sys = (uint32_t)(__ldg(&P.sys_keys[base]) >> 32);
+            const uint32_t lo = __ldg(&P.sys_off[sys]), hi = __ldg(&P.sys_off[sys + 1]);
+            const float4 tail = __ldg(&gnode[lo].tail);  // (a system has at least 256 bodies: inner)
+            const bool first = __float_as_uint(tail.z) == lo && __float_as_uint(tail.w) == hi - lo;
+            root = first ? lo : hi - 1u;
         }
         float bx[BPL], by[BPL], bm[BPL];
         float glox = INFINITY, gloy = INFINITY, ghix = -INFINITY, ghiy = -INFINITY;
@@ -399,7 +399,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
         int sp = 0, nn = 0, nr = 0, nf = 0;
         int turn = 0;  // batches so far
         if (n > 1) {
-            if (lane == 0) S.stack[0] = 0u;
+            if (lane == 0) S.stack[0] = root;
             sp = 1;
         }
         __syncwarp();
@@ -415,14 +415,7 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
             float4 box, tr;
             ldg_half(&gnode[inner ? v : 0u].box, box, tr);
             const uint32_t link = __float_as_uint(tr.z), small = __float_as_uint(tr.w);
-            bool live = inner, spans = false;
-            if (P.num_systems > 0) {
-                const float4 tail = __ldg(&gnode[inner ? v : 0u].tail);
-                const uint32_t f = __float_as_uint(tail.z), e = f + __float_as_uint(tail.w);
-                live = inner & (e > sys_lo) & (f < sys_hi);  // else another system's subtree
-                spans = (f < sys_lo) | (e > sys_hi);         // of several systems: always open
-            }
-            const bool ok = live & !spans & group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2);
+            const bool ok = inner & group_accepts(box, tr.x, tr.y, glox, gloy, ghix, ghiy, th2);
             bool away = false;
             if (FAR) {
                 // far from the group: to its local expansion
@@ -430,10 +423,9 @@ walk_group_kernel(const GNode* __restrict__ gnode, const float4* __restrict__ no
                 const float R2 = __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry));
                 away = ok & (far_rg2 < __fmul_rn(P.far_alpha2, R2));
             }
-            // (a node of several systems holds more bodies than a bucket)
-            const bool bucket = live & !ok & ((small & 255u) <= (uint32_t)P.leaf_size);
-            const bool push = live & !ok & !bucket;
-            const bool range = bucket | (leaf & (v - nm1 >= sys_lo) & (v - nm1 < sys_hi));
+            const bool bucket = inner & !ok & ((small & 255u) <= (uint32_t)P.leaf_size);
+            const bool push = inner & !ok & !bucket;
+            const bool range = bucket | leaf;
             const unsigned mp = __ballot_sync(FULL, push);
             const unsigned mr = __ballot_sync(FULL, range);
             const unsigned mn = __ballot_sync(FULL, ok & !away);
