@@ -9,20 +9,27 @@
 // Design (onesweep, one kernel per 8-bit digit):
 //  - The digit histograms of every pass come from the encode kernel, so each
 //    pass reads its keys exactly once.
-//  - A CTA takes the next tile (512 threads x sort_items keys) from an atomic counter (so lower
-//    tiles are always already running), ranks its keys warp by warp with a
-//    ballot multisplit (stable: item-major, lane-minor = memory order),
-//    publishes its per-digit counts, stages the tile in shared memory in
-//    digit order, and then resolves its global offsets by a decoupled
-//    look-back over the tiles before it, several tiles per round trip.  The
-//    look-back spin is bounded; on giving up it raises kErrLookbackSpin
-//    instead of hanging.
+//  - A CTA takes the next tile (512 threads x sort_items keys) from an atomic
+//    counter (so lower tiles are always already running), ranks its keys warp
+//    by warp (stable: item-major, lane-minor = memory order), publishes its
+//    per-digit counts, stages the tile in shared memory in digit order, and
+//    then resolves its global offsets by a decoupled look-back over the tiles
+//    before it, several tiles per round trip.  The look-back spin is bounded;
+//    on giving up it raises kErrLookbackSpin instead of hanging.
 //  - Staged keys and ids are written out in runs, so global stores are
 //    contiguous per digit.
 //  - Pass 0 does not read ids: it writes the identity permutation of
 //    lbvh.wgsl:68 directly.
 //  - The passes alternate between two buffers and end in the public codes /
 //    ids (an odd number of passes, ensembles only, starts in the others).
+//
+// What bounds it: instruction issue and the chain of a tile's phases, not
+// memory (16.8M 64-bit keys: 2.9 TB/s; wider look-backs, smaller tiles with
+// more CTAs per SM and larger ones with fewer were all slower).  The ranking was
+// half of 165 instructions a warp and 32 keys while it found a digit's lanes by
+// eight ballots; now they meet in a mask in shared memory.  All passes before
+// -> now: 800k 53 -> 43 us, ensembles' 5 passes of 1.2M keys 89 -> 74, 3M 127 ->
+// 104, 64-bit keys 16.8M 1.20 -> 1.10 ms.
 #include <cuda/atomic>
 
 #include "bh_internal.cuh"
@@ -38,24 +45,30 @@ constexpr uint32_t kValueMask = (1u << 30) - 1;
 #endif
 constexpr int kLookBatch = BH_SORT_LOOK_BATCH;  // predecessor tiles read per look-back round
 
-// Exclusive scan over the block (every thread takes part; threads past the
-// 256 digits pass 0, so the digits' prefixes are unaffected by them).
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_tot) {
+// Exclusive scans of two values over the block's 256 digit threads (threads
+// past them pass 0, so the digits' prefixes are unaffected by them).
+__device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint2* s_tot) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
+    uint32_t x = a, y = b;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, x, o), v = __shfl_up_sync(0xFFFFFFFFu, y, o);
+        if (lane >= o) {
+            x += u;
+            y += v;
+        }
     }
-    if (lane == 31) s_tot[warp] = x;
+    if (lane == 31) s_tot[warp] = make_uint2(x, y);
     __syncthreads();
-    uint32_t before = 0;
+    uint32_t bx = 0, by = 0;
 #pragma unroll
     for (int w = 0; w < kRadix / 32; ++w)
-        if (w < warp) before += s_tot[w];
-    __syncthreads();
-    return before + x - v;
+        if (w < warp) {
+            const uint2 t = s_tot[w];
+            bx += t.x;
+            by += t.y;
+        }
+    return make_uint2(bx + x - a, by + y - b);
 }
 
 #ifndef BH_SORT_MIN_BLOCKS
@@ -71,18 +84,24 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
     wait_previous_kernel();
     constexpr int W = kSortThreads / 32;
     constexpr int kSortTile = kSortThreads * kSortItems;
-    __shared__ uint32_t s_whist[W][kRadix];
-    __shared__ uint32_t s_tile_excl[kRadix];
+    __shared__ uint32_t s_whist[W][kRadix];  // a warp's counts, then its first places
     __shared__ uint32_t s_gbase[kRadix];
-    __shared__ uint32_t s_tot[W];
+    __shared__ uint2 s_tot[W];
     __shared__ uint32_t s_tile;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     K* s_keys = reinterpret_cast<K*>(s_dyn);
     uint32_t* s_ids = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
+    // While ranking, the lanes that hold each digit.  (In memory of its own it
+    // took L1 from the walks of other handles that start beside a sort: three
+    // in rotation 8.71 against 8.16 ms a step at 16.8M bodies.)
+    uint32_t(*s_mask)[kRadix] = reinterpret_cast<uint32_t(*)[kRadix]>(s_dyn);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(&scratch->tile_ctr[pass], 1u);
-    for (int i = lane; i < kRadix; i += 32) s_whist[warp][i] = 0;
+    for (int i = lane; i < kRadix; i += 32) {
+        s_whist[warp][i] = 0;
+        s_mask[warp][i] = 0;
+    }
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint32_t seg = tile * kSortTile + (uint32_t)warp * 32u * kSortItems;
@@ -90,83 +109,74 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
 
     K key[kSortItems];
     uint32_t id[kSortItems];
-    uint32_t rank[kSortItems];
+    uint32_t rank[(kSortItems + 1) / 2];  // two 16-bit ranks each
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         uint32_t idx = seg + (uint32_t)k * 32u + (uint32_t)lane;
-        if (idx < n) {
-            key[k] = keys_in[idx];
-            id[k] = FIRST ? idx : ids_in[idx];
-        } else {
-            key[k] = 0;
-            id[k] = 0;
-        }
+        // Places past the end get the largest key: they rank last in the last
+        // tile, and nothing reads that tile's counts.
+        key[k] = ~(K)0;
+        if (idx < n) key[k] = keys_in[idx];
     }
-    // Warp-local stable ranking.  The lanes holding the same digit are found
-    // by eight ballots, one per digit bit (warp multisplit): a constant cost,
-    // where a match instruction slows down with the number of distinct
-    // digits in the warp.
-    const bool full_tile = tile * (uint32_t)kSortTile + (uint32_t)kSortTile <= n;
+    // Warp-local stable ranking: the lanes with a digit meet in its mask.  (Two
+    // ranks a register, ids loaded afterwards: with 64-bit keys all three spill.)
+    const unsigned me = 1u << lane;
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        uint32_t idx = seg + (uint32_t)k * 32u + (uint32_t)lane;
-        bool valid = idx < n;
-        uint32_t d = (uint32_t)(key[k] >> shift) & 0xFFu;
-        unsigned peers = full_tile ? 0xFFFFFFFFu : __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-        for (int bit = 0; bit < kRadixBits; ++bit) {
-            const bool on = (d >> bit) & 1u;
-            const unsigned vote = __ballot_sync(0xFFFFFFFFu, on);
-            peers &= on ? vote : ~vote;
-        }
-        if (!valid) peers = 1u << lane;
-        int leader = __ffs(peers) - 1;
-        uint32_t below = __popc(peers & ((1u << lane) - 1u));
-        uint32_t base = 0;
-        if (valid && lane == leader) {
-            base = s_whist[warp][d];
+        const uint32_t d = (uint32_t)(key[k] >> shift) & 0xFFu;
+        atomicOr(&s_mask[warp][d], me);
+        __syncwarp();
+        const unsigned peers = s_mask[warp][d];
+        const uint32_t base = s_whist[warp][d];
+        __syncwarp();
+        const uint32_t below = __popc(peers & (me - 1u));
+        rank[k / 2] = k & 1 ? rank[k / 2] | (base + below) << 16 : base + below;
+        if (below == 0) {  // the lowest of them
+            s_mask[warp][d] = 0;
             s_whist[warp][d] = base + (uint32_t)__popc(peers);
         }
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        rank[k] = base + below;
         __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+        const uint32_t idx = seg + (uint32_t)k * 32u + (uint32_t)lane;
+        id[k] = FIRST ? idx : idx < n ? ids_in[idx] : 0u;
     }
     __syncthreads();
     // Per digit (threads 0..255): exclusive prefix over warps, and the tile's count.
     static_assert(kSortThreads >= kRadix && kSortThreads % 32 == 0, "one thread per digit");
     const bool digit_thread = tid < kRadix;
     const uint32_t d = digit_thread ? (uint32_t)tid : 0u;
-    uint32_t run = 0;
+    uint32_t tile_cnt = 0;
     if (digit_thread) {
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
-            uint32_t c = s_whist[w][d];
-            s_whist[w][d] = run;
-            run += c;
-        }
+        for (int w = 0; w < W; ++w) tile_cnt += s_whist[w][d];
     }
-    const uint32_t tile_cnt = run;
     // Publish this tile's aggregate (or inclusive prefix for tile 0).
     uint32_t* my_status = status + ((size_t)pass * tiles + tile) * kRadix;
     if (digit_thread) {
         cuda::atomic_ref<uint32_t, cuda::thread_scope_device> a(my_status[d]);
         a.store((tile == 0 ? kFlagPrefix : kFlagAggregate) | tile_cnt, cuda::memory_order_relaxed);
     }
-    const uint32_t tile_excl = block_excl_scan(tile_cnt, s_tot);
-    const uint32_t glob_excl = block_excl_scan(digit_thread ? scratch->hist[pass][d] : 0u, s_tot);
-    if (digit_thread) s_tile_excl[d] = tile_excl;
+    const uint2 before = block_excl_scan2(tile_cnt, digit_thread ? scratch->hist[pass][d] : 0u, s_tot);
+    const uint32_t tile_excl = before.x, glob_excl = before.y;
+    if (digit_thread) {
+        uint32_t run = tile_excl;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const uint32_t c = s_whist[w][d];
+            s_whist[w][d] = run;
+            run += c;
+        }
+    }
     __syncthreads();
     // Stage in digit order before the look-back: the tile's own work is done
     // while the tiles before it finish theirs, so the walk back is shorter.
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        uint32_t idx = seg + (uint32_t)k * 32u + (uint32_t)lane;
-        if (idx < n) {
-            uint32_t dd = (uint32_t)(key[k] >> shift) & 0xFFu;
-            uint32_t p = s_tile_excl[dd] + s_whist[warp][dd] + rank[k];
-            s_keys[p] = key[k];
-            s_ids[p] = id[k];
-        }
+        const uint32_t p = s_whist[warp][(uint32_t)(key[k] >> shift) & 0xFFu] + (k & 1 ? rank[k / 2] >> 16 : rank[k / 2] & 0xFFFFu);
+        s_keys[p] = key[k];
+        s_ids[p] = id[k];
     }
     // Decoupled look-back over earlier tiles, one digit per thread, reading
     // kLookBatch tiles per round trip (nearest first): the values are used up
@@ -212,14 +222,15 @@ onesweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ ids_
         cuda::atomic_ref<uint32_t, cuda::thread_scope_device> a(my_status[d]);
         a.store(kFlagPrefix | (excl + tile_cnt), cuda::memory_order_relaxed);
     }
-    if (digit_thread) s_gbase[d] = glob_excl + excl;
+    // (place in the tile to place in the output: one wrapping addition)
+    if (digit_thread) s_gbase[d] = glob_excl + excl - tile_excl;
     __syncthreads();
     const uint32_t tile_base = tile * kSortTile;
     const uint32_t tile_n = (n - tile_base) < (uint32_t)kSortTile ? (n - tile_base) : (uint32_t)kSortTile;
     for (uint32_t i = (uint32_t)tid; i < tile_n; i += kSortThreads) {
         K kk = s_keys[i];
         uint32_t dd = (uint32_t)(kk >> shift) & 0xFFu;
-        uint32_t dst = s_gbase[dd] + (i - s_tile_excl[dd]);
+        uint32_t dst = s_gbase[dd] + i;
         // Offsets are in range unless a look-back gave up; never write outside.
         if (dst < n) {
             keys_out[dst] = kk;
@@ -236,11 +247,10 @@ int sort_passes(const DeviceBuffers& b) { return b.sort_passes > 0 ? b.sort_pass
 
 // Keys per thread.  Many keys keep a large sort's tiles (and its look-back) few;
 // a small one has fewer tiles than SMs, so it lasts as long as one tile: short
-// tiles below 450k keys.  All passes, 12 / 6 / 3 / 2 / 1 keys (us): 2k bodies
-// 33 / 27 / 21 / 19 / 19, 16k 43 / 35 / 25 / 25 / 25, 100k 45 / 39 / 31 / 31 /
-// 35, 400k 50 / 45 / 45 / 53 / 78, 800k 53 / 55 / 68 / 83 / 132; 64-bit keys
-// 100k 92 / 76 / 58 / 57 / 64, 300k 101 / 85 / 76 / 80 / 119, 1M 136 / 143 /
-// 154 / 193 / 317.
+// tiles below 450k keys.  All passes, 12 / 6 / 3 / 2 keys (us): 2k bodies
+// 31 / 21 / 18 / 16, 16k 33 / 25 / 23 / 20, 100k 35 / 29 / 27 / 27, 400k
+// 41 / 36 / 39 / 49, 500k 41 / 40 / 44 / 57, 800k 45 / 46 / 62 / 77; 64-bit keys
+// 100k 78 / 60 / 51 / 52, 300k 86 / 68 / 70 / 76, 600k 94 / 88 / 107 / 128.
 constexpr int kSmallItems = 3, kLargeItems = 12;
 constexpr uint32_t kSmallSort = 450000;
 static int sort_items(uint32_t n) { return n < kSmallSort ? kSmallItems : kLargeItems; }
@@ -249,9 +259,17 @@ uint32_t sort_tiles(uint32_t n) {
     return (uint32_t)(((uint64_t)n + tile - 1) / tile);
 }
 
+// Dynamic shared memory: the staged tile, and before it the digit masks.
+template <typename K, int ITEMS>
+constexpr size_t sort_smem() {
+    const size_t tile = (size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t));
+    const size_t masks = (size_t)(kSortThreads / 32) * kRadix * sizeof(uint32_t);
+    return tile > masks ? tile : masks;
+}
+
 template <typename K, int ITEMS>
 static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
-    const size_t smem = (size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t));
+    const size_t smem = sort_smem<K, ITEMS>();
     const int passes = sort_passes(b);
     const bool odd = passes & 1;  // the last pass writes codes / ids
     K* kin = (K*)sort_input(b);
@@ -272,7 +290,7 @@ static void sort_impl(const DeviceBuffers& b, cudaStream_t s) {
 
 template <typename K, int ITEMS>
 static cudaError_t set_sort_attributes() {
-    const int smem = (int)((size_t)kSortThreads * ITEMS * (sizeof(K) + sizeof(uint32_t)));
+    const int smem = (int)sort_smem<K, ITEMS>();
     cudaError_t e = cudaFuncSetAttribute(onesweep_kernel<K, ITEMS, true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
