@@ -55,3 +55,34 @@ def test_softenings_and_orders(bh, orc, cfg, bpl):
 @pytest.mark.parametrize("n,alpha", [(300, 0.5), (2500, 0.25), (30011, 0.4)])
 def test_far_batches(bh, orc, n, alpha, bpl):
     _check(bh, orc, n, "colliding-disks", bodiesPerLane=bpl, leafSize=4, farAlpha=alpha)
+
+
+@pytest.mark.parametrize("bpl", [1, 4])
+@pytest.mark.parametrize("kind", ["chain", "pairs", "pile"])
+@pytest.mark.parametrize("n", [3, 33, 300])
+def test_tops_of_uneven_trees(bh, orc, n, kind, bpl):
+    """The top five levels are walked in one step: trees with leaves and long
+    chains among them (bodies at 2^-k, tight pairs of those, one cell holding
+    all but one)."""
+    k = np.arange(n)
+    if kind == "chain":
+        x = 2.0 ** -(k % 15)
+        pos = np.stack([x, x * (1 + k // 15)], 1)
+    elif kind == "pairs":
+        x = 2.0 ** -((k // 2) % 12)
+        pos = np.stack([x + 1e-4 * (k % 2), x * (1 + k // 24)], 1)
+    else:
+        pos = np.stack([1e-3 * (k % 17), 1e-3 * (k // 17)], 1)
+        pos[0] = (1.0, 1.0)
+    sim = bh.Simulation(bh.Config(**BASE, bodiesPerLane=bpl, leafSize=2))
+    sim.setNumBodies(n)
+    pos = pos.astype(np.float32)
+    mass, vel = np.full(n, 1.0 / n, np.float32), np.zeros((n, 2), np.float32)
+    sim.upload(mass, pos, vel)
+    acc = sim.computeAccelerations().astype(np.float64)
+    state = orc.State(orc.params_from_config(sim.config), mass, pos, vel)
+    ref = state.accelerations().astype(np.float64)
+    sim.close()
+    size = np.linalg.norm(ref, axis=1)
+    size = np.maximum(size, np.median(size))
+    assert (np.linalg.norm(acc - ref, axis=1) > 1e-5 * size).mean() <= 0.01
