@@ -10,9 +10,9 @@ bool split_build(uint32_t n, uint32_t debug_flags) {
     return n >= kSplitBuildMin || (n >= 2 && (debug_flags & kDebugSplitBuild));
 }
 
-template <typename K, bool SPLIT>
+template <typename K, bool SPLIT, bool PACK = SPLIT>
 static cudaError_t set_build_attributes() {
-    return cudaFuncSetAttribute(build_fill_kernel<K, SPLIT>,
+    return cudaFuncSetAttribute(build_fill_kernel<K, SPLIT, PACK>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(BuildShared<K, build_block<SPLIT>()>));
 }
@@ -23,6 +23,8 @@ cudaError_t build_init_attributes() {
     cudaError_t e;
     if ((e = set_build_attributes<uint32_t, false>()) != cudaSuccess) return e;
     if ((e = set_build_attributes<uint32_t, true>()) != cudaSuccess) return e;
+    if ((e = set_build_attributes<uint32_t, false, true>()) != cudaSuccess) return e;
+    if ((e = set_build_attributes<uint64_t, false, true>()) != cudaSuccess) return e;
     if ((e = set_build_attributes<uint64_t, false>()) != cudaSuccess) return e;
     return set_build_attributes<uint64_t, true>();
 }
@@ -50,7 +52,8 @@ static void launch_typed(const DeviceBuffers& b, int fp64_levels, cudaStream_t s
     a.err = b.err;
     if (!split_build(b.n, b.debug_flags)) {
         constexpr uint32_t B = build_block<false>();
-        launch_chained(build_fill_kernel<K, false>, (b.n + B - 1) / B, B, sizeof(BuildShared<K, B>), s, a);
+        const auto kernel = b.n < kPackMin ? build_fill_kernel<K, false, false> : build_fill_kernel<K, false, true>;
+        launch_chained(kernel, (b.n + B - 1) / B, B, sizeof(BuildShared<K, B>), s, a);
         return;
     }
     a.frontier = b.frontier;

@@ -119,10 +119,10 @@ struct BuildArgs {
 // at adjacent leaves, so the low levels they create are adjacent in memory.
 // (A persistent variant that hands each finished lane a new leaf measured
 // slower at 16M bodies: its lanes drift apart and its node writes scatter.)
-// Slots per CTA (tree stage, B200): the fused build, 64 / 128 / 256: 800k bodies
-// 102 / 93 / 96 us, 1.5M 170 / 154 / 160, 16k and fewer equal; the split
-// build's local phase takes large ones (16.8M, 256 / 512: 1.52 / 1.43 ms; 4.2M
-// 356 / 374 us).  The frontier climb keeps 256 threads per CTA.
+// Slots per CTA (tree stage, before the packing below): the fused build, 64 /
+// 128 / 256: 800k bodies 102 / 93 / 96 us, 1.5M 170 / 154 / 160, 16k and fewer
+// equal; the split build's local phase takes large ones (16.8M, 256 / 512: 1.52
+// / 1.43 ms; 4.2M 356 / 374 us).  The frontier climb keeps 256 threads per CTA.
 #ifndef BH_BUILD_BLOCK_FUSED
 #define BH_BUILD_BLOCK_FUSED 128
 #endif
@@ -142,6 +142,17 @@ constexpr int build_block() { return SPLIT ? kBuildBlockSplit : kBuildBlockFused
 #endif
 template <bool SPLIT>
 constexpr int build_min_blocks() { return SPLIT ? BH_BUILD_MIN_BLOCKS_SPLIT : 0; }
+// A block's climbers stop after kPackAfter levels and go on in its first warps:
+// after two levels about 5 of a warp's 32 lanes still climb, and every warp went
+// through ~15 levels with them (9-12 lanes an instruction, 43 warp instructions
+// a body).  Tree stage, packed after 1 / 2 / 3 levels / never: 800k bodies 91 /
+// 88 / 88 / 94 us, 4.2M 348 / 345 / 362 / 373, 16.8M 1.35 / 1.36 / 1.39 / 1.44 ms;
+// after 2 / never: 400k 57 / 61 us, 150k 37 / 38, 100k 35 / 35, 70k 35 / 33.  In
+// rotation on three handles the step is 1.5% (800k) and 1% (16.8M) shorter.
+// Below kPackMin the packing's two barriers only lengthen the chain; a runtime
+// switch in one kernel costs that too (16k 25.7 -> 26.2 us a step).
+constexpr int kPackAfter = 2;
+constexpr uint32_t kPackMin = 131072;
 static_assert(kFp64MinBodies > kBuildBlockFused && kFp64MinBodies > kBuildBlockSplit,
               "local nodes must all take the f32 path");
 
@@ -159,6 +170,8 @@ struct BuildShared {
     // {Sxx, Sxy, Syy, body count bits (0: no such node)}, and first slot - B0
     float4 mom[B], box[B], quad[B];
     unsigned short first[B];
+    unsigned short open[B];  // nodes that climb on after the packing (a leaf: B + slot)
+    uint32_t num_open;
 };
 
 // The node a climbing thread currently owns: its slot range, the deltas at
@@ -245,16 +258,17 @@ __device__ __forceinline__ uint32_t make_link(uint32_t gamma, bool left_leaf, bo
     return gamma | (left_leaf ? kLinkLeftLeaf : 0u) | (right_leaf ? kLinkRightLeaf : 0u);
 }
 
-// The block-local climb of one thread (from its leaf `t`): nodes are made and
+// The block-local climb of one thread: nodes are made and
 // exchanged in shared memory only, so a level costs no global store that the
 // fences around the exchange would have to wait for; write_local writes them
 // out afterwards.  Returns true when the node in `c` waits for a split outside
-// the CTA (the thread goes on with it), false when this thread is done.
-template <typename K, int B>
+// the CTA or has climbed LEVELS levels (0: no limit; a thread goes on with it),
+// false when this thread is done.
+template <int LEVELS, typename K, int B>
 __device__ __forceinline__ bool climb_local(const BuildArgs<K>& A, Climb& c, BuildShared<K, B>& S,
                                             uint32_t B0) {
     const uint32_t n = A.n;
-    while (true) {
+    for (int level = 0; LEVELS == 0 || level < LEVELS; ++level) {
         const bool is_left = c.dr > c.dl;
         // boundary (relative) at which this node meets its sibling
         const int q = (int)((is_left ? c.r : c.l - 1u) - B0) + 1;
@@ -301,6 +315,7 @@ __device__ __forceinline__ bool climb_local(const BuildArgs<K>& A, Climb& c, Bui
         S.first[w] = (unsigned short)(pl - B0);
         if (cnt == n) return false;  // the root
     }
+    return true;
 }
 
 // 128-bit relaxed accesses at device scope (single-copy atomic).
@@ -354,7 +369,7 @@ __device__ __forceinline__ bool sibling_word(uint4& got, const uint4* p, uint32_
 // ends, then the sibling's record and the boundary's keys, is three in a row:
 // 3,000-3,300 cycles a level, 13 levels at 2k bodies, 27 at 800k, about 1,300
 // now.  Tree stage: 2k bodies 32 -> 20 us, 16k 39 -> 25, 100k 48 -> 31, 800k
-// 120 -> 93, 16.8M, bound by its local phase, 1.43 ms either way.)
+// 120 -> 93, 16.8M, bound by its local phase, unchanged.)
 template <typename K>
 __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c) {
     const uint32_t n = A.n;
@@ -447,14 +462,16 @@ __device__ __forceinline__ bool climb_step(const BuildArgs<K>& A, Climb& c) {
 // fused build stays resident while one or two of its threads climb the
 // device-scope levels; the split build frees it at the end of its local phase
 // and climbs all frontier nodes side by side, which pays off from a few
-// million bodies up (fused / split: 800k 93 / 105 us, 1.5M 154 / 152, 4.2M
-// 404 / 374, 16.8M 1.51 / 1.43 ms).
+// million bodies up (fused / split, before the packing: 800k 93 / 105 us, 1.5M
+// 154 / 152, 4.2M 404 / 374, 16.8M 1.51 / 1.43 ms).
 // (Climbing the local phase in CTA-wide rounds that pack the remaining
-// nodes into the lowest warps measured slower.  Nor do the random leaf
-// gathers set the pace: with the bodies uploaded in the previous step's
+// nodes into the lowest warps after every level measured slower than packing
+// them once.  Nor do the random leaf gathers set the pace: with the bodies
+// uploaded in the previous step's
 // sorted order, so the gathers run nearly in sequence, the 16.8M-body build
 // took 1.80 against 1.84 ms.)
-template <typename K, bool SPLIT>
+// PACK: the block's climbers go on in its first warps after kPackAfter levels.
+template <typename K, bool SPLIT, bool PACK = SPLIT>
 __global__ void __launch_bounds__(build_block<SPLIT>(), build_min_blocks<SPLIT>())
 build_fill_kernel(const BuildArgs<K> A) {
     constexpr int B = build_block<SPLIT>();
@@ -551,8 +568,53 @@ build_fill_kernel(const BuildArgs<K> A) {
         c.sxx = 0.0f; c.sxy = 0.0f; c.syy = 0.0f;
         c.dm = 0.0; c.dmx = 0.0; c.dmy = 0.0;
     }
+    if (PACK && t == 0) S.num_open = 0;
     __syncthreads();
-    const bool on = active && climb_local<K, B>(A, c, S, B0);
+    bool on;
+    if (PACK) {
+        {
+            const bool open = active && climb_local<kPackAfter>(A, c, S, B0);
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, open);
+            uint32_t at = 0;
+            if (m != 0u && lane == 0) at = atomicAdd(&S.num_open, (uint32_t)__popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (open) {
+                const uint32_t w = (c.dr > c.dl ? c.r : c.l) - B0;  // its Karras index
+                S.open[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] =
+                    (unsigned short)(c.l == c.r ? (uint32_t)B + (c.l - B0) : w);
+            }
+        }
+        __syncthreads();
+        on = (uint32_t)t < S.num_open;
+        if (on) {
+            const uint32_t e = S.open[t];
+            const bool is_leaf = e >= (uint32_t)B;
+            const uint32_t w = is_leaf ? e - (uint32_t)B : e;
+            float4 m, b, q = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t first = w, cnt = 1u;
+            if (is_leaf) {
+                m = S.leaf[w];
+                b = make_float4(m.x, m.y, m.x, m.y);
+            } else {
+                m = S.mom[w];
+                b = S.box[w];
+                q = S.quad[w];
+                first = S.first[w];
+                cnt = __float_as_uint(q.w);
+            }
+            c.l = B0 + first;
+            c.r = c.l + cnt - 1u;
+            c.dl = S.d[first];
+            c.dr = S.d[first + cnt];
+            c.cm = m.z; c.cx = m.x; c.cy = m.y;
+            c.lox = b.x; c.loy = b.y; c.hix = b.z; c.hiy = b.w;
+            c.sxx = q.x; c.sxy = q.y; c.syy = q.z;
+            c.dm = 0.0; c.dmx = 0.0; c.dmy = 0.0;
+            on = climb_local<0>(A, c, S, B0);
+        }
+    } else {
+        on = active && climb_local<0>(A, c, S, B0);
+    }
     __syncthreads();
     // ---- write the CTA's leaves and local nodes, in order ------------------
     if (active) A.node4[nm1 + i] = S.leaf[t];  // leaf (lbvh.wgsl:179-187)
