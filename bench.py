@@ -65,11 +65,11 @@ DEFAULT_WORKLOAD = "colliding-disks-800k"
 FLUSH_BYTES = 256 << 20  # > 126 MB L2
 # DRAM bytes (read + write) of one launch of the dominant kernel (the walk),
 # from one ncu capture of the same workload; the 16.8M point from a capture
-# of its 4.2M-body case (same generator and settings, 1.364 GB) scaled by
+# of its 4.2M-body case (same generator and settings, 1.502 GB) scaled by
 # the bodies processed.
-NCU_WALK_TRAFFIC_BYTES = {"colliding-disks-800k": 72.04e6,  # far-field walk, 128-body groups
-                          "gaussian-mixture-4m": 1.364e9,
-                          "gaussian-mixture-16m": 1.364e9 * 4.0}
+NCU_WALK_TRAFFIC_BYTES = {"colliding-disks-800k": 72.88e6,  # far-field walk, 128-body groups
+                          "gaussian-mixture-4m": 1.502e9,
+                          "gaussian-mixture-16m": 1.502e9 * 4.0}
 # Algorithmic HBM bytes per body and step of the stream stages: encode =
 # position 8 + mass 4 read, key 4|8 + packed leaf record 16 written; sort =
 # first pass key read + key and id written, later passes key and id read and
