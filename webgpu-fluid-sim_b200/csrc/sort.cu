@@ -23,7 +23,7 @@
 //  - The passes alternate between two buffers and end in the public codes /
 //    ids (an odd number of passes, ensembles only, starts in the others).
 //
-// What bounds it: instruction issue and the chain of a tile's phases, not
+// What bounds it: shared-memory wavefronts and the chain of a tile's phases, not
 // memory (16.8M 64-bit keys: 2.9 TB/s; wider look-backs, smaller tiles with
 // more CTAs per SM and larger ones with fewer were all slower).  The ranking was
 // half of 165 instructions a warp and 32 keys while it found a digit's lanes by

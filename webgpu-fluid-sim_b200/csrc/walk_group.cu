@@ -64,12 +64,12 @@
 // lane summing its own; at the end of the group the lanes' sums are reduced
 // and every body evaluates the expansion once (far_field.cuh).
 //
-// What bounds it (B200, 800k colliding disks, 128-body groups, leaf 4): 189M
-// warp instructions at 62% of the issue slots, 24 warps per SM, FMA pipe 47%;
-// the last 14% of the launch is the drain of the last groups.  Walk stage
-// before the branch-free step, id lists, packed far batches and passes over
-// one loop -> now: 800k 389 -> 296 us, 16.8M 7.61 -> 5.59 ms, 64-body groups
-// (ensemble of 64 systems, 1.2M bodies) 584 -> 388 us.
+// What bounds it (B200, 800k colliding disks, 128-body groups, leaf 4): 167M
+// warp instructions at 58% of the issue slots, 20 warps per SM; the last 14% of
+// the launch is the drain of the last groups.  Walk stage before the branch-free
+// step, id lists, packed far batches, passes over one loop and the top in one
+// step -> now: 800k 389 -> 293 us, 16.8M 7.61 -> 5.53 ms, 64-body groups
+// (ensemble of 64 systems, 1.2M bodies) 584 -> 386 us.
 #include "bh_internal.cuh"
 #include "far_field.cuh"
 #include "packed.cuh"
