@@ -1,4 +1,4 @@
-"""The splat's two paths and the tone table at their edges: canvases whose
+"""The splat and the tone table at their edges: canvases whose
 size is no multiple of four (the tone map's vectors), one-pixel and tiny canvases, discs clipped at every side,
 small discs beside large ones, against the oracle's FP64 density (1e-5
 relative, as in the render tests, plus one weight on a disc's rim, 0.1 e^-10,

@@ -49,25 +49,16 @@ struct RenderParams {
 constexpr int kSplatThreads = 256;
 constexpr int kToneThreads = 256;
 
-// density.wgsl:39-97.  Each lane sets up its own body once (centre and radius
-// in pixels, pixel bounds, weight); the setups are shuffled to the lanes that
-// splat.  Small discs (at most kSmallSpan pixels wide and high: all but a
-// scene's few large bodies) go four at a time, eight lanes each, a pixel
-// column per lane, row by row, so a row's adds reach the L2 as one or two
-// 32-byte requests.  Large discs go one after the other, the whole warp in
-// 8 x 4 tiles.  Pixel centres are exactly representable floats and every
-// pixel's weight is computed the same way on both paths: no division or
-// conversion, one hardware exponential.
-// (The warp on one disc at a time spent 78 warp instructions on a 5 x 5 pixel
-// disc, mostly idle lanes and shuffles, and was bound by their issue.  Now the
-// L2's requests bound it: a frame of 800k bodies at 1920 x 1080, with the tone
-// table below, 91 -> 48 us; zoomed out until all of them share a few thousand
-// pixels, where the adds meet each other, 109-138 us before and 112 now.  A
-// disc per lane with one 16-byte vector reduction per four pixels needs as
-// many requests and meets itself more often: 48 and 135 us; scalar reductions
-// 89 and 249 us.  16 / 4 / 2 blocks per SM: 46 / 50 / 60 and 110 / 137 / 139.)
-constexpr int kSmallSpan = 8;
-constexpr uint32_t kSplatBlocksPerSm = 8;
+// density.wgsl:39-97, one warp per 32 bodies.  Each lane sets up its own
+// body once (centre and radius in pixels, pixel bounds, weight) and the warp
+// then splats the 32 bodies one after the other, the setup of each shuffled
+// from its lane.  The lanes cover the body's pixel rectangle in 8 x 4 tiles,
+// with integer pixel indices and exactly representable float pixel centres
+// stepped by additions: no division or conversion per pixel, one hardware
+// exponential per covered pixel.  (Small discs four to a warp, eight lanes
+// each, took a frame of 800k bodies from 62 to 34 us, but add to a pixel in another order: 0
+// to 5 more of an image's 8.3M bytes differed than between two runs of this
+// order, whose float atomics already differ in 0 to 2.)
 __global__ void __launch_bounds__(kSplatThreads)
 splat_kernel(const float2* __restrict__ pos, const float* __restrict__ radius_mul, uint32_t n,
              const RenderParams P, float* __restrict__ density) {
@@ -109,50 +100,28 @@ splat_kernel(const float2* __restrict__ pos, const float* __restrict__ radius_mu
             inv_r = __frcp_rn(R);
             bw = __fmul_rn(rm > 1.0f ? 0.1f : 0.02f, zoom_scale);  // density.wgsl:90-95
         }
-        // uv and r^2 = |uv|^2; discard outside the disc (density.wgsl:73-78);
-        // w = exp(-k r^2), k = 10 (density.wgsl:81-82): the hardware exponential,
-        // relative error ~1e-6 over r^2 in [0, 1]
-        auto splat = [](float* px, float ux2, float uy2, float w) {
-            const float r2 = __fadd_rn(ux2, uy2);
-            if (!(r2 > 1.0f)) atomicAdd(px, __fmul_rn(w, __expf(__fmul_rn(-10.0f, r2))));
-        };
-        auto square = [](float c, float centre, float ir) {
-            const float u = __fmul_rn(__fsub_rn(c, centre), ir);
-            return __fmul_rn(u, u);
-        };
-        const bool drawn = ia <= ib;
-        const bool small = drawn && ib - ia < kSmallSpan && jb - ja < kSmallSpan;
-        const unsigned smalls = __ballot_sync(FULL, small);
-        const int gx = lane & 7, gy = lane >> 3;
-#pragma unroll 1
-        for (int it = 0; it < 8; ++it) {
-            const int k = 4 * it + gy;
+        const int cnt = (n - base) < 32u ? (int)(n - base) : 32;
+        for (int k = 0; k < cnt; ++k) {
             const int kia = __shfl_sync(FULL, ia, k), kib = __shfl_sync(FULL, ib, k);
             const int kja = __shfl_sync(FULL, ja, k), kjb = __shfl_sync(FULL, jb, k);
-            const float kcx = __shfl_sync(FULL, cpx, k), kcy = __shfl_sync(FULL, cpy, k);
-            const float kir = __shfl_sync(FULL, inv_r, k), kbw = __shfl_sync(FULL, bw, k);
-            const int i = kia + gx;
-            if (((smalls >> k) & 1u) && i <= kib) {
-                const float ux2 = square((float)i + 0.5f, kcx, kir);
-                float yc = (float)kja + 0.5f;
-                float* px = density + (size_t)kja * P.w + i;
-                for (int j = kja; j <= kjb; ++j, yc = __fadd_rn(yc, 1.0f), px += P.w)
-                    splat(px, ux2, square(yc, kcy, kir), kbw);
-            }
-        }
-        for (unsigned large = __ballot_sync(FULL, drawn && !small); large; large &= large - 1u) {
-            const int k = __ffs(large) - 1;
-            const int kia = __shfl_sync(FULL, ia, k), kib = __shfl_sync(FULL, ib, k);
-            const int kja = __shfl_sync(FULL, ja, k), kjb = __shfl_sync(FULL, jb, k);
+            if (kia > kib) continue;  // nothing on screen (uniform)
             const float kcx = __shfl_sync(FULL, cpx, k), kcy = __shfl_sync(FULL, cpy, k);
             const float kir = __shfl_sync(FULL, inv_r, k), kbw = __shfl_sync(FULL, bw, k);
             float yc = (float)(kja + ty) + 0.5f;
             for (int j = kja + ty; j <= kjb; j += 4, yc = __fadd_rn(yc, 4.0f)) {
-                const float uy2 = square(yc, kcy, kir);
+                // uv and r^2 = |uv|^2; discard outside the disc (density.wgsl:73-78)
+                const float uy = __fmul_rn(__fsub_rn(yc, kcy), kir);
+                const float uy2 = __fmul_rn(uy, uy);
                 float* row = density + (size_t)j * P.w;
                 float xc = (float)(kia + tx) + 0.5f;
-                for (int i = kia + tx; i <= kib; i += 8, xc = __fadd_rn(xc, 8.0f))
-                    splat(&row[i], square(xc, kcx, kir), uy2, kbw);
+                for (int i = kia + tx; i <= kib; i += 8, xc = __fadd_rn(xc, 8.0f)) {
+                    const float ux = __fmul_rn(__fsub_rn(xc, kcx), kir);
+                    const float r2 = __fadd_rn(__fmul_rn(ux, ux), uy2);
+                    if (r2 > 1.0f) continue;
+                    // w = exp(-k r^2), k = 10 (density.wgsl:81-82): the hardware
+                    // exponential, relative error ~1e-6 over r^2 in [0, 1]
+                    atomicAdd(&row[i], __fmul_rn(kbw, __expf(__fmul_rn(-10.0f, r2))));
+                }
             }
         }
     }
@@ -380,7 +349,7 @@ extern "C" int bh_renderer_frame(bh_renderer* r) {
     if (v.n > 0) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
-        uint32_t blocks = (uint32_t)sms * bh::kSplatBlocksPerSm;
+        uint32_t blocks = (uint32_t)sms * 8u;
         const uint32_t need = (v.n + bh::kSplatThreads - 1) / bh::kSplatThreads;
         if (blocks > need) blocks = need;
         bh::splat_kernel<<<blocks, bh::kSplatThreads, 0, v.stream>>>(v.pos, v.radius, v.n, P,
